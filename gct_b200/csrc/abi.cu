@@ -1349,9 +1349,16 @@ gct_status gct_forward_project(const gct_ct_geom *geom, const gct_vol_geom *vol,
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const int nr = vol3d ? static_cast<int>(geom->det_col.num_samples) : 1;
+        // the copies of the grid that the rays read; without memory for them the grid is read as it is
+        DevBuf<float> copies;
+        try {
+            copies.alloc(static_cast<size_t>(gct::forward_scratch_floats(box)), "grid copies");
+        } catch (const gct::GctError &) {
+        }
         gct::launch_forward(dv.p, kind, static_cast<int>(geom->num_views), nr,
                             static_cast<int>(geom->det_row.num_samples), geom->det_row.sampling_width,
-                            vol3d ? geom->det_col.sampling_width : 1.0, vol_dev, box, step_vox, proj_dev, sms, s);
+                            vol3d ? geom->det_col.sampling_width : 1.0, vol_dev, copies.p, box, step_vox, proj_dev, sms,
+                            s);
         cuda_check(cudaGetLastError(), "forward projector launch");
         cuda_check(cudaStreamSynchronize(s), "forward projection");
     });

@@ -7,11 +7,18 @@
 //   arc / cylinder : origin S, direction cos(g) e_w + sin(g) e_u + (t / SDD) e_v
 // with u = (c - c0) du, v = (r - r0) dv (src/cuda/geom/coord_trans_proj.cuh:142-150, the
 // inverse of DCSToPCS).
+#include <climits>
+
 #include "../../include/gct_fdk.h"
 #include "project.hpp"
 
 namespace gct {
 namespace {
+
+// Grids up to this size (64 KB) are read as they are: their calls take longer to allocate and fill
+// the copies than the copies save (25 x 25 x 24 voxels, 36 views of 48 x 40: 0.69 ms a call against
+// 0.75 with copies; 32 x 32 x 31, 90 views of 64 x 64: 0.75 against 0.84).
+constexpr long long kCopyVoxels = 1 << 14;
 
 struct Ray {
     double o[3];
@@ -118,58 +125,275 @@ __device__ __forceinline__ float trilinear(const float *__restrict__ vol, int nx
     return acc;
 }
 
-__global__ void forward_kernel(const ProjView *__restrict__ views, int kind, int nv, int nr, int nc,
-                               double du, double dv, const float *__restrict__ vol, VolBox box,
-                               float step_vox, float *__restrict__ out)
+// Forward projection: midpoint sums of trilinear samples every step_vox voxel lengths between a
+// ray's two crossings of the grid's outer faces (half a voxel outside the outermost centres).
+//
+// Ray setup is FP64 and gives the sample positions as x(s) = x0 + s dx per axis in voxel-index
+// units. The samples whose taps all lie in the grid (solved for s per axis, kEdge voxels inside the
+// taps' range) run without range checks in chunks of kChunk samples: the chunk's start is evaluated
+// in FP64 and split into a whole voxel, which goes into the chunk's base pointer, and a remainder;
+// the samples are FP32 steps from it, so a position is within 4e-6 voxels of its FP64 value for steps
+// of half a voxel (a direct FP32 position at voxel 128 is within 8e-6). The floor is one add that
+// rounds down at 1.5 * 2^23 (its bits are the voxel offset). The samples at the ray's two ends take
+// the range-checked path.
+//
+// The warp marches its rays in step along axis 1: lane l takes sample k + o_l in iteration k, o_l
+// chosen so that every lane is at the same plane of axis 1 (rays that enter through different faces
+// start at different depths). The 32 lanes' taps then lie in one or two rows of the grid.
+//
+// Bound by the latency and the L1 wavefronts of the gathers (3.3 lines per request of (z, z + 1)
+// pairs), so four blocks per SM (64 registers, the ray setup spills) beat three (80 registers: 20.1 ms)
+// and two with twice the loads in flight (18.7 ms). 192^3 grid, 180 views of 384 x 288, half-voxel
+// steps (7.7e9 samples): 70.7 ms with FP64 positions and range checks per sample, 54 ms without
+// those, 33 ms with the exchanged copy, 19.3 ms marching in step, 16.5 ms with packed pairs and the
+// masked ends. Chunks of 64 samples: 18.8 ms (more masked samples at the rays' ends).
+constexpr int kChunk = 32;
+constexpr double kEdge = 1.0 / 1024.0;
+constexpr float kFloorShift = 12582912.0f;  // 1.5 * 2^23
+constexpr int kFloorBits = 0x4B400000;
+
+__device__ __forceinline__ float2 lerp2(float2 a, float2 b, float2 f)
 {
-    const long long total = static_cast<long long>(nv) * nr * nc;
-    for (long long idx = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; idx < total;
-         idx += static_cast<long long>(gridDim.x) * blockDim.x) {
-        const int c = static_cast<int>(idx % nc);
-        const long long vr = idx / nc;
-        const int r = static_cast<int>(vr % nr);
-        const int v = static_cast<int>(vr / nr);
+    return __ffma2_rn(f, __ffma2_rn(a, make_float2(-1.f, -1.f), b), a);
+}
+
+// Sum of one ray; every lane of the warp calls it (`on` false: the lane has no ray). `grid` holds the
+// box's voxels (PAIRS: each with the voxel of the next plane); the range-checked samples read `vol`,
+// in which x and y are the other way round where `swapped`. Off: the type of byte offsets into the
+// grid (32 bits below 4 GB: one register, added to a uniform address).
+template <bool PLANAR, bool PAIRS, class Off>
+__device__ __forceinline__ float forward_ray(const Ray &ray, bool on, const float *__restrict__ vol,
+                                             const float *__restrict__ grid, bool swapped, const VolBox &box,
+                                             float step_vox)
+{
+    constexpr int NA = PLANAR ? 2 : 3;
+    const int n[3] = {box.nx, box.ny, box.nz};
+    const double dn = sqrt(ray.d[0] * ray.d[0] + ray.d[1] * ray.d[1] + ray.d[2] * ray.d[2]);
+    double dir[NA];
+    // slab intersection with the voxel-centre box extended by half a voxel
+    double t0 = -1e300, t1 = 1e300;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        dir[a] = ray.d[a] / dn;
+        const double lo = box.lo[a] - 0.5 * box.w[a], hi = box.hi[a] + 0.5 * box.w[a];
+        if (fabs(dir[a]) < 1e-15) {
+            if (ray.o[a] < lo || ray.o[a] > hi) on = false;
+            continue;
+        }
+        const double ta = (lo - ray.o[a]) / dir[a], tb = (hi - ray.o[a]) / dir[a];
+        t0 = fmax(t0, fmin(ta, tb));
+        t1 = fmin(t1, fmax(ta, tb));
+    }
+    const double wmin = PLANAR ? fmin(box.w[0], box.w[1]) : fmin(box.w[0], fmin(box.w[1], box.w[2]));
+    const double h = static_cast<double>(step_vox) * wmin;
+    const long long ns = on && t1 > t0 ? static_cast<long long>(ceil((t1 - t0) / h)) : 0;
+    // x(s) = x0 + s dx; samples [sa, sb) have every tap inside the grid
+    double x0[NA], dx[NA], fa = 0.0, fb = static_cast<double>(ns) - 1.0, dmax = 0.0;
+#pragma unroll
+    for (int a = 0; a < NA; ++a) {
+        x0[a] = (ray.o[a] + (t0 + 0.5 * h) * dir[a] - box.lo[a]) / box.w[a];
+        dx[a] = h * dir[a] / box.w[a];
+        dmax = fmax(dmax, fabs(dx[a]));
+        const double lo = kEdge - x0[a], hi = (n[a] - 1.0 - kEdge) - x0[a];
+        if (fabs(dx[a]) * static_cast<double>(ns) < 0.5 * kEdge) {  // stays where it starts
+            if (!(lo + 0.5 * kEdge <= 0.0 && hi - 0.5 * kEdge >= 0.0)) fb = -1.0;
+        } else {
+            fa = fmax(fa, (dx[a] > 0.0 ? lo : hi) / dx[a]);
+            fb = fmin(fb, (dx[a] > 0.0 ? hi : lo) / dx[a]);
+        }
+    }
+    long long sa = ns, sb = ns;
+    if (fb >= fa && dmax <= 1.0 && ns < (1LL << 30) && static_cast<long long>(box.nx) * box.ny <= (1LL << 25)) {
+        sa = static_cast<long long>(ceil(fa));
+        sb = static_cast<long long>(floor(fb)) + 1;
+        if (sb <= sa) sa = sb = ns;
+    }
+    float sum = 0.f;
+    auto checked = [&](long long s) {
+        const double f = static_cast<double>(s);
+        const float x = static_cast<float>(fma(f, dx[0], x0[0])), y = static_cast<float>(fma(f, dx[1], x0[1]));
+        const float z = PLANAR ? 0.f : static_cast<float>(fma(f, dx[NA - 1], x0[NA - 1]));
+        sum += swapped ? trilinear(vol, box.ny, box.nx, box.nz, y, x, z) : trilinear(vol, box.nx, box.ny, box.nz, x, y, z);
+    };
+    for (long long s = 0; s < sa; ++s) checked(s);
+    // iterations [ka, kb) of this lane in the warp's march
+    const bool run = sb > sa;
+    const unsigned runners = __ballot_sync(0xffffffffu, run);
+    int ka = INT_MAX, kb = INT_MIN, shift = 0;
+    if (runners) {
+        const double yref = __shfl_sync(0xffffffffu, x0[1], __ffs(runners) - 1);
+        if (run) {
+            if (fabs(dx[1]) > 0.1) {
+                const double o = rint((yref - x0[1]) / dx[1]);
+                if (fabs(o) < 1e6) shift = static_cast<int>(o);
+            }
+            ka = static_cast<int>(sa) - shift;
+            kb = static_cast<int>(sb) - shift;
+        }
+    }
+    const int kend = __reduce_max_sync(0xffffffffu, kb);
+    const int sy = box.nx, sz = box.nx * box.ny;
+    const float d[3] = {static_cast<float>(dx[0]), static_cast<float>(dx[1]), PLANAR ? 0.f : static_cast<float>(dx[NA - 1])};
+    // the taps of a voxel offset: row addresses, the same for every lane (offsets in bytes)
+    constexpr int kVox = PAIRS ? 8 : 4;
+    const char *const b00 = reinterpret_cast<const char *>(grid), *const b01 = b00 + static_cast<long long>(kVox) * sy,
+                      *const b10 = b00 + static_cast<long long>(kVox) * sz,
+                      *const b11 = b10 + static_cast<long long>(kVox) * sy;
+    auto at = [](const char *row, Off o) { return __ldg(reinterpret_cast<const float *>(row + o)); };
+    auto at2 = [](const char *row, Off o) { return __ldg(reinterpret_cast<const float2 *>(row + o)); };
+    float2 sum2 = make_float2(0.f, 0.f);
+    for (int k0 = __reduce_min_sync(0xffffffffu, ka); k0 < kend; k0 += kChunk) {
+        if (ka >= k0 + kChunk || kb <= k0) continue;  // no sample of this lane in the chunk
+        float r[3] = {0.f, 0.f, 0.f};
+        long long c[3] = {0, 0, 0};
+#pragma unroll
+        for (int a = 0; a < NA; ++a) {
+            const double xb = fma(static_cast<double>(k0 + shift), dx[a], x0[a]), fl = floor(xb);
+            c[a] = static_cast<int>(fl);
+            r[a] = static_cast<float>(xb - fl);
+        }
+        // byte offset of the chunk's first voxel, less what the bits of the shifted floors add (both
+        // modulo 2^32 in the 32-bit form: the sum is the offset of a voxel of the grid)
+        const Off base = static_cast<Off>(kVox * ((c[2] * box.ny + c[1]) * box.nx + c[0] -
+                                                  static_cast<long long>(kFloorBits) * (1LL + sy + (PLANAR ? 0 : sz))));
+        // samples k and k + 1 as packed pairs at (FP32) chunk positions fk
+        auto pair = [&](float2 fk) -> float2 {
+            float2 f[NA];
+            Off o0 = base, o1 = base;
+#pragma unroll
+            for (int a = 0; a < NA; ++a) {
+                const float2 x = __ffma2_rn(fk, make_float2(d[a], d[a]), make_float2(r[a], r[a]));
+                const float2 t = __fadd2_rd(x, make_float2(kFloorShift, kFloorShift));  // floor(x) in the low bits
+                f[a] = __ffma2_rn(__fadd2_rn(t, make_float2(-kFloorShift, -kFloorShift)), make_float2(-1.f, -1.f), x);
+                const Off st = a == 0 ? kVox : static_cast<Off>(static_cast<long long>(kVox) * (a == 1 ? sy : sz));
+                o0 += static_cast<Off>(__float_as_int(t.x)) * st;
+                o1 += static_cast<Off>(__float_as_int(t.y)) * st;
+            }
+            if constexpr (PAIRS) {
+                // (z, z + 1) pairs of four taps per sample
+                const float2 p00 = at2(b00, o0), p01 = at2(b00 + 8, o0), p10 = at2(b01, o0), p11 = at2(b01 + 8, o0);
+                const float2 q00 = at2(b00, o1), q01 = at2(b00 + 8, o1), q10 = at2(b01, o1), q11 = at2(b01 + 8, o1);
+                const float2 x0 = make_float2(f[0].x, f[0].x), y0 = make_float2(f[1].x, f[1].x);
+                const float2 x1 = make_float2(f[0].y, f[0].y), y1 = make_float2(f[1].y, f[1].y);
+                const float2 e0 = lerp2(lerp2(p00, p01, x0), lerp2(p10, p11, x0), y0);
+                const float2 e1 = lerp2(lerp2(q00, q01, x1), lerp2(q10, q11, x1), y1);
+                return lerp2(make_float2(e0.x, e1.x), make_float2(e0.y, e1.y), f[NA - 1]);
+            } else {
+                const float2 v00 = make_float2(at(b00, o0), at(b00, o1)), v01 = make_float2(at(b00 + 4, o0), at(b00 + 4, o1));
+                const float2 v10 = make_float2(at(b01, o0), at(b01, o1)), v11 = make_float2(at(b01 + 4, o0), at(b01 + 4, o1));
+                const float2 e = lerp2(lerp2(v00, v01, f[0]), lerp2(v10, v11, f[0]), f[1]);
+                if constexpr (PLANAR) return e;
+                const float2 w00 = make_float2(at(b10, o0), at(b10, o1)), w01 = make_float2(at(b10 + 4, o0), at(b10 + 4, o1));
+                const float2 w10 = make_float2(at(b11, o0), at(b11, o1)), w11 = make_float2(at(b11 + 4, o0), at(b11 + 4, o1));
+                return lerp2(e, lerp2(lerp2(w00, w01, f[0]), lerp2(w10, w11, f[0]), f[1]), f[NA - 1]);
+            }
+        };
+        const float lo = static_cast<float>(max(ka - k0, 0)), hi = static_cast<float>(min(kb - k0, kChunk) - 1);
+        float2 fk = make_float2(0.f, 1.f);
+        if (__all_sync(__activemask(), lo == 0.f && hi == kChunk - 1.f)) {
+#pragma unroll 1
+            for (int k = 0; k < kChunk; k += 2, fk = __fadd2_rn(fk, make_float2(2.f, 2.f))) sum2 = __fadd2_rn(sum2, pair(fk));
+        } else {  // some ray starts or ends in the chunk: its other samples repeat its first or last one, unsummed
+#pragma unroll 1
+            for (int k = 0; k < kChunk; k += 2, fk = __fadd2_rn(fk, make_float2(2.f, 2.f))) {
+                const float2 fc = make_float2(fminf(fmaxf(fk.x, lo), hi), fminf(fmaxf(fk.y, lo), hi));
+                const float2 e = pair(fc);
+                sum2.x += fc.x == fk.x ? e.x : 0.f;
+                sum2.y += fc.y == fk.y ? e.y : 0.f;
+            }
+        }
+    }
+    sum += sum2.x + sum2.y;
+    for (long long s = sb; s < ns; ++s) checked(s);
+    return sum * static_cast<float>(h);
+}
+
+// Whether a view's rays run more along x than along y (its central direction, one answer per view).
+__device__ __forceinline__ bool along_x(const ProjView &pv, int kind)
+{
+    double x = pv.ew[0], y = pv.ew[1];
+    if (kind == GCT_GEOM_PARALLEL_1D || kind == GCT_GEOM_PARALLEL_2D || kind == GCT_GEOM_CONE_PARALLEL)
+        sincos(pv.extra, &y, &x);
+    return fabs(x) > fabs(y);
+}
+template <class T>
+__device__ __forceinline__ void swap2(T *a)
+{
+    const T t = a[0];
+    a[0] = a[1];
+    a[1] = t;
+}
+
+// Blocks take tiles of bx x by detector pixels of one view (bx by = 256, bx >= 32), in turn. The
+// rays of a warp lie side by side across their direction, so a warp's taps are neighbours along the
+// grid axis that the rays cross. Views whose rays run along x read `along`, the grid with x and y
+// exchanged (NULL for none), where those neighbours are contiguous; in the grid itself they are nx
+// voxels apart and every gather would touch 32 cache lines.
+template <bool PLANAR, bool PAIRS, class Off>
+__global__ void __launch_bounds__(256, 4) forward_kernel(const ProjView *__restrict__ views, int kind, int nv, int nr,
+                                                         int nc, double du, double dv, const float *__restrict__ vol,
+                                                         const float *__restrict__ across,
+                                                         const float *__restrict__ along, VolBox box, float step_vox,
+                                                         int bx, float *__restrict__ out)
+{
+    const int by = 256 / bx, tc = (nc + bx - 1) / bx, tr = (nr + by - 1) / by;
+    const long long tiles = static_cast<long long>(nv) * tr * tc;
+    for (long long tile = blockIdx.x; tile < tiles; tile += gridDim.x) {
+        const int v = static_cast<int>(tile / (static_cast<long long>(tr) * tc));
+        const int rem = static_cast<int>(tile - static_cast<long long>(v) * tr * tc);
+        const int r = (rem / tc) * by + threadIdx.x / bx, c = (rem % tc) * bx + threadIdx.x % bx;
+        const bool on = r < nr && c < nc;
         Ray ray = make_ray(views[v], kind, du, dv, c, r);
-        if (box.planar) {
+        if (PLANAR) {
             ray.o[2] = box.lo[2];
             ray.d[2] = 0.0;
         }
-        const double dn = sqrt(ray.d[0] * ray.d[0] + ray.d[1] * ray.d[1] + ray.d[2] * ray.d[2]);
-        double dir[3] = {ray.d[0] / dn, ray.d[1] / dn, ray.d[2] / dn};
-        // slab intersection with the voxel-centre box extended by half a voxel
-        double t0 = -1e300, t1 = 1e300;
-        bool hit = true;
-        for (int a = 0; a < 3; ++a) {
-            if (box.planar && a == 2) continue;
-            const double lo = box.lo[a] - 0.5 * box.w[a], hi = box.hi[a] + 0.5 * box.w[a];
-            if (fabs(dir[a]) < 1e-15) {
-                if (ray.o[a] < lo || ray.o[a] > hi) hit = false;
-                continue;
-            }
-            double ta = (lo - ray.o[a]) / dir[a], tb = (hi - ray.o[a]) / dir[a];
-            if (ta > tb) {
-                const double tmp = ta;
-                ta = tb;
-                tb = tmp;
-            }
-            t0 = fmax(t0, ta);
-            t1 = fmin(t1, tb);
+        VolBox b = box;
+        const bool swapped = along && along_x(views[v], kind);
+        if (swapped) {  // x and y exchanged throughout
+            swap2(ray.o);
+            swap2(ray.d);
+            swap2(b.lo);
+            swap2(b.hi);
+            swap2(b.w);
+            b.nx = box.ny;
+            b.ny = box.nx;
         }
-        float sum = 0.f;
-        if (hit && t1 > t0) {
-            const double wmin = box.planar ? fmin(box.w[0], box.w[1]) : fmin(box.w[0], fmin(box.w[1], box.w[2]));
-            const double h = static_cast<double>(step_vox) * wmin;
-            const long long ns = static_cast<long long>(ceil((t1 - t0) / h));
-            for (long long s = 0; s < ns; ++s) {
-                const double t = t0 + (static_cast<double>(s) + 0.5) * h;
-                const float x = static_cast<float>((ray.o[0] + t * dir[0] - box.lo[0]) / box.w[0]);
-                const float y = static_cast<float>((ray.o[1] + t * dir[1] - box.lo[1]) / box.w[1]);
-                const float z = box.planar ? 0.f : static_cast<float>((ray.o[2] + t * dir[2] - box.lo[2]) / box.w[2]);
-                sum += trilinear(vol, box.nx, box.ny, box.nz, x, y, z);
+        const float sum = forward_ray<PLANAR, PAIRS, Off>(ray, on, vol, swapped ? along : across, swapped, b, step_vox);
+        if (on) out[(static_cast<long long>(v) * nr + r) * nc + c] = sum;
+    }
+}
+
+// The grid's copies for the rays, in one pass over 32 x 32 tiles (32 x 8 threads): along[z][x][y] =
+// vol[z][y][x]; PAIRS: along and across as (z, z + 1) pairs (zero past the last plane).
+template <bool PAIRS>
+__global__ void arrange_grid_kernel(const float *__restrict__ vol, int nx, int ny, int nz, float *__restrict__ across,
+                                    float *__restrict__ along)
+{
+    __shared__ float tile[2][32][33];
+    const int tx = (nx + 31) / 32, ty = (ny + 31) / 32;
+    const long long tiles = static_cast<long long>(tx) * ty * nz, plane = static_cast<long long>(nx) * ny;
+    for (long long t = blockIdx.x; t < tiles; t += gridDim.x) {
+        const long long z = t / (static_cast<long long>(tx) * ty);
+        const int rem = static_cast<int>(t - z * tx * ty), x0 = (rem % tx) * 32, y0 = (rem / tx) * 32;
+        for (int k = threadIdx.y; k < 32; k += 8) {
+            if (y0 + k >= ny || x0 + threadIdx.x >= nx) continue;
+            const long long at = z * plane + static_cast<long long>(y0 + k) * nx + x0 + threadIdx.x;
+            const float v = __ldg(vol + at), w = PAIRS && z + 1 < nz ? __ldg(vol + at + plane) : 0.f;
+            tile[0][k][threadIdx.x] = v;
+            if (PAIRS) {
+                tile[1][k][threadIdx.x] = w;
+                reinterpret_cast<float2 *>(across)[at] = make_float2(v, w);
             }
-            sum *= static_cast<float>(h);
         }
-        out[idx] = sum;
+        __syncthreads();
+        for (int k = threadIdx.y; k < 32; k += 8) {
+            if (x0 + k >= nx || y0 + threadIdx.x >= ny) continue;
+            const long long at = z * plane + static_cast<long long>(x0 + k) * ny + y0 + threadIdx.x;
+            if (PAIRS) reinterpret_cast<float2 *>(along)[at] = make_float2(tile[0][threadIdx.x][k], tile[1][threadIdx.x][k]);
+            else along[at] = tile[0][threadIdx.x][k];
+        }
+        __syncthreads();
     }
 }
 
@@ -188,15 +412,40 @@ void launch_phantom(const ProjView *views, int kind, int nv, int nr, int nc, dou
 }
 
 void launch_forward(const ProjView *views, int kind, int nv, int nr, int nc, double du, double dv,
-                    const float *vol, const VolBox &box, float step_vox, float *out, int num_sms,
+                    const float *vol, float *scratch, const VolBox &box, float step_vox, float *out, int num_sms,
                     cudaStream_t s)
 {
-    const long long total = static_cast<long long>(nv) * nr * nc;
-    long long grid = (total + 255) / 256;
-    if (grid > static_cast<long long>(num_sms) * 32) grid = static_cast<long long>(num_sms) * 32;
+    const long long voxels = static_cast<long long>(box.nx) * box.ny * box.nz;
+    const float *across = vol, *along = nullptr;
+    if (scratch) {
+        float *ac = box.planar ? nullptr : scratch, *al = box.planar ? scratch : scratch + 2 * voxels;
+        long long grid = static_cast<long long>((box.nx + 31) / 32) * ((box.ny + 31) / 32) * box.nz;
+        if (grid > static_cast<long long>(num_sms) * 64) grid = static_cast<long long>(num_sms) * 64;
+        if (box.planar)
+            arrange_grid_kernel<false><<<static_cast<unsigned>(grid), dim3(32, 8), 0, s>>>(vol, box.nx, box.ny, box.nz, ac, al);
+        else
+            arrange_grid_kernel<true><<<static_cast<unsigned>(grid), dim3(32, 8), 0, s>>>(vol, box.nx, box.ny, box.nz, ac, al);
+        if (!box.planar) across = ac;
+        along = al;
+    }
+    const int bx = nr >= 8 ? 32 : nr >= 4 ? 64 : nr >= 2 ? 128 : 256, by = 256 / bx;
+    long long grid = static_cast<long long>(nv) * ((nr + by - 1) / by) * ((nc + bx - 1) / bx);
+    if (grid > static_cast<long long>(num_sms) * 64) grid = static_cast<long long>(num_sms) * 64;
     if (grid < 1) grid = 1;
-    forward_kernel<<<static_cast<unsigned>(grid), 256, 0, s>>>(views, kind, nv, nr, nc, du, dv, vol, box,
-                                                               step_vox, out);
+    auto go = [&](auto kern) {
+        kern<<<static_cast<unsigned>(grid), 256, 0, s>>>(views, kind, nv, nr, nc, du, dv, vol, across, along, box,
+                                                         step_vox, bx, out);
+    };
+    if (box.planar) go(forward_kernel<true, false, long long>);
+    else if (!scratch) go(forward_kernel<false, false, long long>);
+    else if (8 * voxels < (1LL << 32)) go(forward_kernel<false, true, unsigned>);
+    else go(forward_kernel<false, true, long long>);
+}
+
+long long forward_scratch_floats(const VolBox &box)
+{
+    const long long voxels = static_cast<long long>(box.nx) * box.ny * box.nz;
+    return voxels <= kCopyVoxels ? 0 : voxels * (box.planar ? 1 : 4);
 }
 
 }  // namespace gct

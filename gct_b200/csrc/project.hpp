@@ -28,8 +28,11 @@ void launch_phantom(const ProjView *views, int kind, int nv, int nr, int nc, dou
                     const gct_ellipsoid *ell, int ne, bool planar, float *out, int num_sms,
                     cudaStream_t s);
 
+// scratch: room for forward_scratch_floats() floats, the copies of the grid that the rays read (made
+// here on the stream), or NULL: the rays read the grid itself, slower.
+long long forward_scratch_floats(const VolBox &box);
 void launch_forward(const ProjView *views, int kind, int nv, int nr, int nc, double du, double dv,
-                    const float *vol, const VolBox &box, float step_vox, float *out, int num_sms,
+                    const float *vol, float *scratch, const VolBox &box, float step_vox, float *out, int num_sms,
                     cudaStream_t s);
 
 }  // namespace gct
