@@ -145,24 +145,12 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
     for (int v = 0; v < p->nv; ++v) wscale[v] = dtheta * vd[v].bp_const;
     std::vector<double> coefs64;
     std::vector<float> coefs = gct::bp_coefficients(p->geom, p->vol, vd, wscale, &p->z_affine, &coefs64);
-    // 1D parallel kind: transpose, so that the detector coordinate u(x, y) = u0 + ui x + uj y becomes
-    // the row coordinate v(i, k) = v0 + vi i + vk k of a one-column detector and image rows run
-    // along the backprojector's z loop
-    p->t1d = kind == GCT_GEOM_PARALLEL_1D;
+    p->rows = !gct::is_2d_detector(kind) &&
+              (p->opts.storage == GCT_STORAGE_F32 || p->family == gct::Family::Affine ||
+               (p->family == gct::Family::Projective && p->opts.filter == GCT_FILTER_FFT));
     p->kx = static_cast<int>(vol->nx);
-    p->ky = p->t1d ? 1 : static_cast<int>(vol->ny);
-    p->kz = p->t1d ? static_cast<int>(vol->ny) : static_cast<int>(vol->nz);
-    if (p->t1d) {
-        for (int v = 0; v < static_cast<int>(g->num_views); ++v) {
-            float *c = &coefs[static_cast<size_t>(v) * gct::kCoefPerView];
-            const float u0 = c[0], ui = c[1], uj = c[2];
-            c[0] = c[1] = c[2] = 0.0f;  // the single detector column
-            c[3] = u0;
-            c[6] = ui;
-            c[4] = uj;
-            c[7] = 0.0f;
-        }
-    }
+    p->ky = static_cast<int>(vol->ny);
+    p->kz = static_cast<int>(vol->nz);
 
     std::vector<float4> fview(p->nv);
     for (int v = 0; v < p->nv; ++v)
@@ -243,17 +231,17 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
     // with 8 x 16 blocks for FP16 quads (2047 GUPS; 8 voxels: 1855, 32: 1543) and with 4 x 16 blocks
     // for FP32 quads (1466 GUPS; 8 voxels on 4 x 32: 1425)
     const bool f16 = p->opts.storage == GCT_STORAGE_F16;
-    // the transposed 1D parallel kind loops over image rows: 16 rows per thread, 128 x 1 blocks
-    const int zpt3d = 16;
-    p->zpt = p->opts.z_per_thread > 0 ? p->opts.z_per_thread : ((vol3d || p->t1d) ? zpt3d : 1);
+    // row-pair plans have a fixed shape of their own (rows.cu); their options are checked all the same
+    const bool par1d = kind == GCT_GEOM_PARALLEL_1D;
+    p->zpt = p->opts.z_per_thread > 0 ? p->opts.z_per_thread : (vol3d ? 16 : 1);
     if (p->zpt != 1 && p->zpt != 2 && p->zpt != 4 && p->zpt != 8 && p->zpt != 16)
         gct::fail(GCT_ERR_INVALID_ARG, "z_per_thread must be 1, 2, 4, 8 or 16");
-    p->bx = p->opts.block_x > 0 ? p->opts.block_x : (p->t1d ? 128 : vol3d ? (f16 ? 8 : 4) : 32);
-    p->by = p->opts.block_y > 0 ? p->opts.block_y : (p->t1d ? 1 : vol3d ? 16 : 8);
+    p->bx = p->opts.block_x > 0 ? p->opts.block_x : (par1d ? 128 : vol3d ? (f16 ? 8 : 4) : 32);
+    p->by = p->opts.block_y > 0 ? p->opts.block_y : (par1d ? 1 : vol3d ? 16 : 8);
     if (p->bx * p->by > 256 || p->bx * p->by < 32)
         gct::fail(GCT_ERR_INVALID_ARG, "backprojection block must hold 32..256 threads");
-    // quarter-turn form: the z-affine column kernels (not the transposed 1D kind, whose kernel
-    // grid is x by image rows); at most 8 voxels per thread, since each thread keeps four columns.
+    // quarter-turn form: the z-affine column kernels and the fans over row pairs (not the 1D parallel
+    // kind); at most 8 voxels per thread, since each thread keeps four columns.
     // Measured on B200 (512^3, 720 views): FP16 quads 34.4 ms against 47.2 ms for the plain kernel
     // (8 voxels per thread, 2 x 32 blocks; 4 x 16: 35.5, 8 x 16: 36.6, 4 voxels: 36.9); FP32 quads
     // 88 ms against 64 ms (a 64-byte partner group per voxel), so AUTO takes it for FP16 storage
@@ -262,12 +250,12 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
     if (so != GCT_SYMMETRY_AUTO && so != GCT_SYMMETRY_OFF && so != GCT_SYMMETRY_ON)
         gct::fail(GCT_ERR_INVALID_ARG, "unknown symmetry option");
     const bool want = so == GCT_SYMMETRY_ON || (so == GCT_SYMMETRY_AUTO && f16);
-    if (want && !p->t1d && (p->family == gct::Family::Affine || p->z_affine))
+    if (want && !par1d && (p->family == gct::Family::Affine || p->z_affine))
         p->sym = gct::quarter_turn_symmetry(kind, coefs64, static_cast<unsigned>(p->nv), vol->nx, vol->ny,
                                             static_cast<unsigned>(p->kz));
     // z-mirror form of the column kernels (plans without the quarter-turn form, whose kernel has
     // its own sharing): each thread takes a segment of the lower half and its mirror voxels
-    if (want && !p->sym && !p->t1d && !p->spiral && p->zpt % 2 == 0 &&
+    if (want && !p->sym && !p->rows && !p->spiral && p->zpt % 2 == 0 &&
         (p->family == gct::Family::Affine || (p->family == gct::Family::Projective && p->z_affine)))
         p->mirror = gct::z_mirror_symmetry(kind, coefs64, static_cast<unsigned>(p->nv), static_cast<unsigned>(p->nr),
                                            vol->nx, vol->ny, static_cast<unsigned>(p->kz));
@@ -277,7 +265,7 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
     if (p->mirror && p->opts.z_per_thread <= 0) p->zpt = 8;
     // quarter-turn stacks are prepared through FP32 rows (prepare_partners); the GEMM filter has
     // its row buffer already
-    if (p->sym && !p->ybuf.p)
+    if (p->sym && !p->rows && !p->ybuf.p)
         p->ybuf.alloc(static_cast<size_t>(p->nv) * p->nr * p->nc, "filtered rows of quarter-turn stacks");
     if (p->spiral) {
         // one slice per thread along z: each slice has its own window of views
@@ -364,7 +352,7 @@ void run_filter_gemm(gct_fdk_plan *p, const float *proj, void *out, const float 
     const long long row0 = static_cast<long long>(vb) * p->nr, rows = static_cast<long long>(vc) * p->nr;
     split_rows(p, proj, vb, vc, 0, s, fused_scales);
     gct::GemmLaunch gl = gemm_launch(p);
-    if (mode == gct::kOutQuadF16 && quarter == 0 && !p->t1d && p->nc % 2 == 0 &&
+    if (mode == gct::kOutQuadF16 && quarter == 0 && p->nc % 2 == 0 &&
         reinterpret_cast<uintptr_t>(out) % 16 == 0 && gct::gemm_quad_tiles(rows, 1) >= p->num_sms) {
         // view-major FP16 quads straight from the GEMM's epilogue
         gl.quads = out;
@@ -381,6 +369,12 @@ void run_filter_gemm(gct_fdk_plan *p, const float *proj, void *out, const float 
     gl.ldy = p->nc;
     cuda_check(gct::launch_toeplitz_gemm(gl, p->num_sms, s), "Toeplitz GEMM launch");
     if (mode == gct::kOutPlainF32) return;
+    if (p->rows) {
+        gct::launch_row_pairs(gl.Y, vb, vc, p->nc, p->kind == GCT_GEOM_PARALLEL_1D,
+                              mode == gct::kOutRowsF16 ? vscale : nullptr, out, p->num_sms, s);
+        cuda_check(cudaGetLastError(), "row pair kernel launch");
+        return;
+    }
     gct::QuadArgs qa;
     qa.Y = gl.Y;
     qa.ldy = p->nc;
@@ -388,7 +382,6 @@ void run_filter_gemm(gct_fdk_plan *p, const float *proj, void *out, const float 
     qa.nv = vc;
     qa.nr = p->nr;
     qa.nc = p->nc;
-    qa.t1d = p->t1d ? 1 : 0;
     qa.vscale = (mode == gct::kOutQuadF16) ? vscale : nullptr;
     qa.out = out;
     qa.quarter = quarter;
@@ -399,7 +392,7 @@ void run_filter_gemm(gct_fdk_plan *p, const float *proj, void *out, const float 
 
 }  // namespace
 
-// `out` is the view-0 address of the output; `vscale` (FP16 quads only) the view-0 scales;
+// `out` is the view-0 address of the output; `vscale` (FP16 stacks only) the view-0 scales;
 // `quarter` the quad_layout of a quad output. `fused_scales` (Toeplitz form only, amax zeroed by
 // the caller): the split pass also finds the view maxima and the scales follow it.
 void run_filter(gct_fdk_plan *p, const float *proj, void *out, const float *vscale, int mode, int quarter, int vb,
@@ -431,8 +424,7 @@ void run_filter(gct_fdk_plan *p, const float *proj, void *out, const float *vsca
         fa.v0 = vb;
         fa.quarter = quarter;
     }
-    fa.vscale = (mode == gct::kOutQuadF16) ? vscale + vb : nullptr;
-    fa.t1d = (p->t1d && mode != gct::kOutPlainF32) ? 1 : 0;
+    fa.vscale = (mode == gct::kOutQuadF16 || mode == gct::kOutRowsF16) ? vscale + vb : nullptr;
     gct::launch_filter_fft(fa, static_cast<int>(p->L), p->num_sms, s);
     cuda_check(cudaGetLastError(), "filter kernel launch");
 }
@@ -441,21 +433,21 @@ gct::BpArgs bp_args(const gct_fdk_plan *p, const StackRef &st, float *vol, int v
 {
     gct::BpArgs ba;
     ba.quads = st.quads;
-    // the quad grid per view holds (nr + 4) x (nc + 4) entries in either orientation
-    ba.qpitch = p->t1d ? gct::kT1dPitch : p->nc + 2 * gct::kQuadPad;
-    ba.qview = static_cast<long long>(p->nr + 2 * gct::kQuadPad) * (p->nc + 2 * gct::kQuadPad);
+    ba.qpitch = p->nc + 2 * gct::kQuadPad;
+    ba.qview = static_cast<long long>(p->rows ? 1 : p->nr + 2 * gct::kQuadPad) * ba.qpitch;
     ba.coefs = p->coefs.p;
     ba.vinv = st.vinv;
     ba.v_begin = v_begin;
     ba.v_count = v_count;
-    ba.quarter = st.quarter;
+    ba.quarter = p->rows && p->sym ? p->nv / 4 : st.quarter;
+    if (p->rows) ba.sym = p->sym;
     ba.slice_views = p->slice_views.p;
     ba.vol = vol;
     ba.nx = p->kx;
     ba.ny = p->ky;
     ba.nz = p->kz;
-    ba.umax = static_cast<float>(p->t1d ? 1 : p->nc);
-    ba.vmax = static_cast<float>(p->t1d ? p->nc : p->nr);
+    ba.umax = static_cast<float>(p->nc);
+    ba.vmax = static_cast<float>(p->nr);
     return ba;
 }
 
@@ -465,7 +457,7 @@ namespace {
 // into the most parts (chunks of at least 8 views) whose blocks fit two whole waves.
 int split_chunk(const gct_fdk_plan *p, long long blocks, int per_sm, int views)
 {
-    if (p->kz != 1 || p->spiral || p->t1d || blocks <= 0 || per_sm <= 0 || views < 16) return 0;
+    if (p->kz != 1 || p->spiral || blocks <= 0 || per_sm <= 0 || views < 16) return 0;
     const long long wave = static_cast<long long>(p->num_sms) * per_sm;
     if (blocks >= wave) return 0;
     const long long parts = std::min<long long>(2 * wave / blocks, views / 8);
@@ -506,6 +498,11 @@ void run_backproject(gct_fdk_plan *p, const StackRef &st, float *vol, int v_begi
     }
     gct::BpArgs ba = bp_args(p, st, vol, v_begin, v_count);
     ba.accumulate = accumulate ? 1 : 0;
+    if (p->rows) {
+        gct::launch_backproject_rows(ba, static_cast<int>(p->family), p->opts.storage, p->num_sms, s);
+        cuda_check(cudaGetLastError(), "backprojection kernel launch");
+        return;
+    }
     ba.mirror = (p->mirror && st.quarter == 0) ? 1 : 0;  // view-major stacks only
     const long long blocks = static_cast<long long>((p->kx + p->bx - 1) / p->bx) * ((p->ky + p->by - 1) / p->by);
     const int chunk =
@@ -552,7 +549,7 @@ void check_range(const gct_fdk_plan *p, uint32_t vb, uint32_t vc)
 void *plan_workspace(gct_fdk_plan *p, void *workspace)
 {
     if (workspace) return workspace;
-    if (!p->work.p) p->work.alloc(p->workspace_bytes(), "plan workspace");
+    if (!p->work.p) p->work.alloc(p->stack_bytes(), "plan workspace");
     return p->work.p;
 }
 
@@ -576,7 +573,8 @@ void prepare(gct_fdk_plan *p, const float *proj, const StackRef &st, int vb, int
     const bool fuse = f16 && p->opts.filter != GCT_FILTER_FFT;  // the split pass finds the maxima
     if (fuse) cuda_check(cudaMemsetAsync(st.amax + vb, 0, sizeof(float) * vc, s), "view maxima reset");
     else if (f16) view_scales(p, proj, st, vb, vc, s);
-    run_filter(p, proj, st.quads, st.vscale, f16 ? gct::kOutQuadF16 : gct::kOutQuadF32, st.quarter, vb, vc, s,
+    const int mode = p->rows ? (f16 ? gct::kOutRowsF16 : gct::kOutRowsF32) : f16 ? gct::kOutQuadF16 : gct::kOutQuadF32;
+    run_filter(p, proj, st.quads, st.vscale, mode, st.quarter, vb, vc, s,
                fuse ? &st : nullptr);
 }
 
@@ -751,7 +749,7 @@ void execute_host_budget(gct_fdk_plan *p, const float *proj_host, float *vol_hos
         // puts this chunk at the start of the slot and of the chunk stack
         StackRef st;
         st.quads = reinterpret_cast<unsigned char *>(reinterpret_cast<uintptr_t>(ws) -
-                                                     static_cast<uintptr_t>(vb) * p->view_bytes());
+                                                     static_cast<uintptr_t>(vb) * p->view_stride());
         if (f16) {
             st.amax = scales - vb;
             st.vscale = scales + chunk - vb;
@@ -1172,7 +1170,7 @@ void execute_noalloc(gct_fdk_plan *p, const float *proj, float *vol, cudaStream_
 {
     if (!proj || !vol) gct::fail(GCT_ERR_INVALID_ARG, "NULL projection or volume pointer");
     // per view: its quads and, for FP16 storage, three floats (maximum, scale, inverse scale)
-    const size_t quads_per_view = p->view_bytes();
+    const size_t quads_per_view = p->view_stride();
     const size_t scales_per_view = p->opts.storage == GCT_STORAGE_F16 ? 3 * sizeof(float) : 0;
     const size_t per_view = quads_per_view + scales_per_view;
     if (per_view + 256 > GCT_NOALLOC_SCRATCH_BYTES)

@@ -216,9 +216,8 @@ __device__ __forceinline__ int box_class(const float *c, float i0, float i1, flo
         float u, va, vb;
         if (FAMILY == 0) {
             u = fmaf(c[2], fj, fmaf(c[1], fi, c[0]));
-            const float V = fmaf(c[7], fj, fmaf(c[6], fi, c[3]));
-            va = fmaf(c[4], k0, V);
-            vb = fmaf(c[4], k1, V);
+            va = fmaf(c[4], k0, c[3]);
+            vb = fmaf(c[4], k1, c[3]);
         } else {
             const float D = fmaf(c[10], fj, fmaf(c[9], fi, c[8]));
             if (!(D > 0.0f)) return kBoxMixed;
@@ -311,9 +310,9 @@ __device__ __forceinline__ void bp_column(const BpArgs &a, int i, int j, int k0,
             const S *view = ES == 1 ? quads + v * a.qview : quads + ((v % a.quarter) * a.qview * 4 + v / a.quarter);
             constexpr int es = ES;
             if (FAMILY == 0) {
-                // parallel kinds: u = u0 + ui i + uj j, v = v0 + vi i + vj j + vk k, constant weight
+                // parallel kinds: u = u0 + ui i + uj j, v = v0 + vk k, constant weight
                 const float u = fmaf(c[2], fj, fmaf(c[1], fi, c[0]));
-                const float v0 = fmaf(c[4], fk0, fmaf(c[7], fj, fmaf(c[6], fi, c[3])));
+                const float v0 = fmaf(c[4], fk0, c[3]);
                 column_dispatch<L, ZPT, MIRROR>(view, es, a.qpitch, u, v0, c[4], a.umax, a.vmax, ConstWeight{c[5]},
                                                 acc, cls, MIRROR ? &accm : nullptr);
             } else if (FAMILY == 1) {
@@ -621,7 +620,7 @@ __device__ __forceinline__ void sym_rotation(const BpArgs &a, const float *c, fl
     if (cls == kBoxOff) return;
     if (FAMILY == 0) {
         const float u = fmaf(c[2], fj, fmaf(c[1], fi, c[0]));
-        const float v0 = fmaf(c[4], fk0, fmaf(c[7], fj, fmaf(c[6], fi, c[3])));
+        const float v0 = fmaf(c[4], fk0, c[3]);
         column4_dispatch<L, ZPT, K>(group0, a.qpitch, u, v0, c[4], a.umax, a.vmax,
                                     ConstWeight4{{w.x, w.y, w.z, w.w}}, acc, cls);
     } else if (FAMILY == 1) {
@@ -997,6 +996,7 @@ int queue_blocks_per_sm(int storage, int zclass)
 {
     int n = 0;
     cudaError_t e;
+    if (zclass == kQueueRowsClass) return rows_queue_blocks_per_sm(storage);
     if (zclass == kQueueSymClass)
         e = storage == 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bp_queue_sym_kernel<QuadF32>, kQueueThreads, 0)
                          : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, bp_queue_sym_kernel<QuadF16>, kQueueThreads, 0);
@@ -1012,6 +1012,10 @@ int queue_blocks_per_sm(int storage, int zclass)
 void launch_backproject_queue(const BpItem *items, const BpWork *work, int n_work, int *counter, int storage,
                               int zclass, int grid, cudaStream_t s)
 {
+    if (zclass == kQueueRowsClass) {
+        launch_rows_queue(items, work, n_work, counter, storage, grid, s);
+        return;
+    }
     if (zclass == kQueueSymClass) {
         if (storage == 0) bp_queue_sym_kernel<QuadF32><<<grid, kQueueThreads, 0, s>>>(items, work, n_work, counter);
         else bp_queue_sym_kernel<QuadF16><<<grid, kQueueThreads, 0, s>>>(items, work, n_work, counter);

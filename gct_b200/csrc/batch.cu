@@ -38,6 +38,12 @@ BpItem make_item(const gct_fdk_plan *p, const StackRef &st, float *vol, const Ti
     it.bx = c.bx;
     it.by = c.by;
     it.vps = c.vps;
+    if (p->rows) {
+        it.tiles_x = (p->kx + kRowsTileX - 1) / kRowsTileX;
+        it.tiles_y = (p->ky + kRowsTileY - 1) / kRowsTileY;
+        it.tiles_z = 1;
+        return it;
+    }
     if (st.quarter) {  // quarter-turn item: tiles of first-quadrant columns
         if (!sym_queue_zpt_ok(c.zpt))
             fail(GCT_ERR_INVALID_ARG, "quarter-turn queue tiles hold 8 voxels per thread (1 for 2D images)");
@@ -54,7 +60,10 @@ BpItem make_item(const gct_fdk_plan *p, const StackRef &st, float *vol, const Ti
 }
 
 int item_views(const gct_fdk_plan *p, const StackRef &st) { return st.quarter ? st.quarter : p->nv; }
-int item_class(const StackRef &st, const TileConfig &c) { return st.quarter ? kQueueSymClass : queue_class(c.zpt); }
+int item_class(const gct_fdk_plan *p, const StackRef &st, const TileConfig &c)
+{
+    return p->rows ? kQueueRowsClass : st.quarter ? kQueueSymClass : queue_class(c.zpt);
+}
 
 long long item_tiles(const BpItem &it) { return static_cast<long long>(it.tiles_x) * it.tiles_y * it.tiles_z; }
 
@@ -72,10 +81,10 @@ TileConfig default_config(const gct_fdk_plan *p, bool quarter_turn)
         c.zpt = vol3d(p) ? 8 : 1;
         c.bx = vol3d(p) ? 8 : 16;
         c.by = vol3d(p) ? 32 : 16;
-    } else if (p->ky == 1 && vol3d(p)) {  // one row of columns (the transposed 1D parallel kind)
-        c.bx = 256;
-        c.by = 1;
-        c.zpt = 16;
+    } else if (p->rows) {  // rows.cu: 8 pixels per thread along y
+        c.zpt = 1;
+        c.bx = kRowsTileX;
+        c.by = kQueueThreads / kRowsTileX;
     } else if (!vol3d(p)) {
         c.zpt = 1;
         c.bx = 32;
@@ -87,14 +96,12 @@ TileConfig default_config(const gct_fdk_plan *p, bool quarter_turn)
 namespace {
 
 // Candidate (zpt, block) shapes; views per stage is tuned afterwards for the best shape.
-std::vector<TileConfig> shape_candidates(bool three_d, bool one_row, bool quarter_turn)
+std::vector<TileConfig> shape_candidates(bool three_d, bool quarter_turn)
 {
     std::vector<TileConfig> c;
     if (quarter_turn) {
         for (auto b : {std::make_pair(8, 32), std::make_pair(4, 64), std::make_pair(16, 16), std::make_pair(32, 8)})
             c.push_back({three_d ? 8 : 1, b.first, b.second, 32});
-    } else if (one_row) {
-        for (int zpt : {8, 16}) c.push_back({zpt, 256, 1, 32});
     } else if (three_d) {
         for (int zpt : {8, 16})
             for (auto b : {std::make_pair(8, 32), std::make_pair(16, 16), std::make_pair(32, 8)})
@@ -118,7 +125,7 @@ struct QueueScratch {
 double time_config(const gct_fdk_plan *p, const StackRef &st, float *vol, const TileConfig &c, int num_sms,
                    QueueScratch &sc, cudaStream_t s)
 {
-    const int zc = item_class(st, c);
+    const int zc = item_class(p, st, c);
     const int grid = std::max(1, queue_blocks_per_sm(p->opts.storage, zc)) * num_sms;
     const BpItem it = make_item(p, st, vol, c);
     const int nvt = std::min(item_views(p, st), st.quarter ? 16 : 64);
@@ -171,11 +178,14 @@ Tuned autotune(const gct_fdk_plan *p, const StackRef &st, float *vol, int num_sm
     }
     QueueScratch sc;
     Tuned best;
-    for (const TileConfig &c : shape_candidates(vol3d(p), p->ky == 1 && vol3d(p), st.quarter > 0)) {
+    const std::vector<TileConfig> shapes =
+        p->rows ? std::vector<TileConfig>{default_config(p, false)} : shape_candidates(vol3d(p), st.quarter > 0);
+    for (const TileConfig &c : shapes) {
         const double ups = time_config(p, st, vol, c, num_sms, sc, s);
         if (ups > best.ups) best = {c, ups};
     }
     for (int vps : {16, 64}) {
+        if (p->rows) break;  // planar tiles stage a fixed number
         TileConfig c = best.cfg;
         c.vps = vps;
         const double ups = time_config(p, st, vol, c, num_sms, sc, s);
@@ -298,7 +308,7 @@ void build_batch(gct_fdk_batch *b, const gct_batch_item *items, uint32_t n, cons
         it->plan = src.plan;
         it->proj = src.proj_dev;
         it->vol = src.vol_dev;
-        it->ws.alloc(src.plan->workspace_bytes(), "batch item workspace");
+        it->ws.alloc(src.plan->stack_bytes(), "batch item workspace");
         // quarter-turn plans keep their interleaved partner stacks and run in the quarter-turn queue
         it->st = stack_of(src.plan, it->ws.p, false);
         b->items.push_back(std::move(it));
@@ -339,7 +349,7 @@ void build_batch(gct_fdk_batch *b, const gct_batch_item *items, uint32_t n, cons
     // work queues: items by decreasing cost; an item whose single tile costs more than an even
     // share of the queue over 8 entries per block is split into view chunks (atomic adds)
     auto queue_of = [&](const gct_fdk_batch::Item &it) {
-        return (it.plan->opts.storage == GCT_STORAGE_F16 ? 1 : 0) * kQueueClasses + item_class(it.st, it.cfg);
+        return (it.plan->opts.storage == GCT_STORAGE_F16 ? 1 : 0) * kQueueClasses + item_class(it.plan, it.st, it.cfg);
     };
     for (int q = 0; q < 2 * kQueueClasses; ++q) {
         auto &Q = b->queue[q];

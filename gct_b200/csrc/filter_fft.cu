@@ -338,23 +338,14 @@ __device__ __forceinline__ void write_quad_row(const FilterArgs &a, int v, int q
     }
 }
 
-// Transposed quad grid of view v of a one-row detector from its filtered row y (shared, padded
-// as above).
+// Row pairs of view v from its filtered row y (shared, padded as above).
 template <int MODE>
-__device__ __forceinline__ void write_quads_t1d(const FilterArgs &a, int v, const float *y, int t, int nthr)
+__device__ __forceinline__ void write_row_pairs(const FilterArgs &a, int v, const float *y, int t, int nthr)
 {
-    const int nc = a.nc, rows = nc + 2 * kQuadPad;
-    const long long base = static_cast<long long>(v) * rows * kT1dPitch;
-    for (int e = t; e < rows * kT1dPitch; e += nthr) {
-        const int r = e / kT1dPitch, c = e % kT1dPitch - kQuadPad;  // y[r - 2] is shared entry r
-        const float tp = y[r], bt = y[r + 1];
-        if (c == 0)
-            store_quad<MODE>(a.out, base + e, tp, 0.0f, bt, 0.0f);
-        else if (c == -1)
-            store_quad<MODE>(a.out, base + e, 0.0f, tp, 0.0f, bt);
-        else
-            store_quad<MODE>(a.out, base + e, 0.0f, 0.0f, 0.0f, 0.0f);
-    }
+    const int pitch = a.nc + 2 * kQuadPad;
+    const bool centred = a.kind == GCT_GEOM_PARALLEL_1D;
+    for (int e = t; e < pitch; e += nthr)
+        store_row_pair<MODE == kOutRowsF16>(a.out, static_cast<long long>(v) * pitch + e, y[e], y[e + 1], centred);
 }
 
 // Loads, weights and packs detector rows a (real part) and b (imaginary part) at columns t + T m;
@@ -645,8 +636,8 @@ __global__ void __launch_bounds__(Fft<LOG2L>::T, fft_min_blocks<LOG2L>())
                 const int v = h ? pr.vb : pr.va;
                 if (v < 0) continue;
                 const float *y = h ? yb : ya;
-                if (a.t1d) {
-                    write_quads_t1d<MODE>(a, a.v0 + v, y, t, T);
+                if constexpr (MODE == kOutRowsF32 || MODE == kOutRowsF16) {
+                    write_row_pairs<MODE>(a, a.v0 + v, y, t, T);
                 } else {
                     write_quad_row<MODE>(a, a.v0 + v, -2, nullptr, nullptr, t, T);
                     write_quad_row<MODE>(a, a.v0 + v, -1, nullptr, y, t, T);
@@ -727,11 +718,12 @@ void launch_mode(const FilterArgs &a, int num_sms, cudaStream_t s)
         cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem));
         kern<<<static_cast<unsigned>(grid), F::T, smem, s>>>(a, seg, nseg);
     };
-    if (a.nr == 1) {
+    constexpr bool kRows = MODE == kOutRowsF32 || MODE == kOutRowsF16;  // one-row detectors only
+    if (kRows || a.nr == 1) {
         if (!bulk) go(filter_fft_kernel<LOG2L, MODE, false, true, false>);
         else if (half) go(filter_fft_kernel<LOG2L, MODE, true, true, true>);
         else go(filter_fft_kernel<LOG2L, MODE, false, true, true>);
-    } else {
+    } else if constexpr (!kRows) {
         if (!bulk) go(filter_fft_kernel<LOG2L, MODE, false, false, false>);
         else if (half) go(filter_fft_kernel<LOG2L, MODE, true, false, true>);
         else go(filter_fft_kernel<LOG2L, MODE, false, false, true>);
@@ -744,6 +736,8 @@ void launch_log2(const FilterArgs &a, int num_sms, cudaStream_t s)
     switch (a.mode) {
         case kOutPlainF32: launch_mode<LOG2L, kOutPlainF32>(a, num_sms, s); break;
         case kOutQuadF32: launch_mode<LOG2L, kOutQuadF32>(a, num_sms, s); break;
+        case kOutRowsF32: launch_mode<LOG2L, kOutRowsF32>(a, num_sms, s); break;
+        case kOutRowsF16: launch_mode<LOG2L, kOutRowsF16>(a, num_sms, s); break;
         default: launch_mode<LOG2L, kOutQuadF16>(a, num_sms, s); break;
     }
 }

@@ -75,7 +75,6 @@ struct QuadArgs {
     const float *vscale = nullptr;
     void *out = nullptr;       // quads of the full stack
     int quarter = 0;           // quad_layout (kernels.hpp)
-    int t1d = 0;               // one-row detector: transposed quad grid (kernels.hpp, kT1dPitch)
     int *err = nullptr;        // plan status word: kQuadWaitTimeout when a row copy timed out
 };
 constexpr int kQuadWaitTimeout = 0x200;

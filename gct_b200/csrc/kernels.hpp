@@ -9,7 +9,7 @@ namespace gct {
 // Zero padding (entries per side) of the bilinear-quad layout of filtered projections.
 constexpr int kQuadPad = 2;
 
-enum FilterOut : int { kOutPlainF32 = 0, kOutQuadF32 = 1, kOutQuadF16 = 2 };
+enum FilterOut : int { kOutPlainF32 = 0, kOutQuadF32 = 1, kOutQuadF16 = 2, kOutRowsF32 = 3, kOutRowsF16 = 4 };
 
 struct FilterArgs {
     const float *proj = nullptr;   // [nv][nr][nc] raw projections
@@ -20,11 +20,10 @@ struct FilterArgs {
     const float *parker = nullptr; // [nv][nc]
     const float2 *H = nullptr;     // [L] filter spectrum, scaled by 1/L
     int mode = kOutPlainF32;
-    void *out = nullptr;           // plain: rows of views [0, nv); quads: view 0 of the stack (quad_layout)
-    int v0 = 0;                    // quads: stack index of the first view filtered
+    void *out = nullptr;           // plain: rows of views [0, nv); quads, row pairs: view 0 of the stack
+    int v0 = 0;                    // quads, row pairs: stack index of the first view filtered
     int quarter = 0;               // quads: quad_layout's quarter
-    const float *vscale = nullptr; // per-view output scale for quads (nullable = 1)
-    int t1d = 0;                   // one-row detectors: write the transposed quad grid (t1d_quad_layout)
+    const float *vscale = nullptr; // per-view output scale for quads and row pairs (nullable = 1)
     int *err = nullptr;            // plan status word: kFftWaitTimeout when an input copy timed out
 };
 
@@ -47,12 +46,13 @@ __host__ __device__ inline void quad_layout(long long v, long long qview, int qu
     }
 }
 
-// Transposed quads of a one-row detector (1D parallel kind): the nc cells become the rows of a
-// one-column image, so that the backprojector's row coordinate runs along the image's y axis (an
-// affine function of the thread's loop index) and its column coordinate is the constant 0. Grid
-// per view: (nc + 4) rows x 5 columns, entry (r, c) for r in [-2, nc + 2), c in [-2, 3); the quad
-// at column 0 holds (y[r], 0, y[r + 1], 0) and at column -1 (0, y[r], 0, y[r + 1]).
-constexpr int kT1dPitch = 1 + 2 * kQuadPad;
+// Row pairs: the stack of planar kinds (1D parallel, fan line, fan arc), whose views are one row. Entry c of a view, for c in [-2, nc + 2), is (y[c], y[c + 1] - y[c]), for the
+// parallel kind ((y[c] + y[c + 1]) / 2, y[c + 1] - y[c]), with zeros outside the row, as float2 or half2
+// (scaled as the quads); views follow each other nc + 4 entries apart. With FP16 storage the
+// fans keep quads in two cases: arcs, whose blends round the column fraction to half precision, which
+// turns last-bit differences of the angle into differences of a 2048th sample, so they stay with
+// atan2f and the quarter-turn kernel that shares it between four updates; and lines with a Toeplitz
+// filter, whose GEMM writes its quads itself.
 
 // Fused cosine + Parker weighting, zero padding, FFT convolution with the ramp filter and the
 // epilogue into the requested layout. L is the power-of-two FFT length (256 to 8192).
@@ -108,6 +108,14 @@ void launch_backproject(const BpArgs &a, int family, int storage, bool z_affine,
 // view and accumulates them into the column's four quarter-turn images from the four partner views.
 void launch_backproject_sym(const BpArgs &a, int family, int storage, int zpt, int bx, int by, cudaStream_t s);
 
+// Planar kinds over row pairs (rows.cu): views [a.v_begin, a.v_begin + a.v_count) into the image.
+// a.quads, a.qview: the pairs and the entries per view; a.sym, a.quarter: quarter-turn plans, whose
+// view v takes its coordinates from base view v mod quarter at the turned pixel (view-major all the same).
+void launch_backproject_rows(const BpArgs &a, int family, int storage, int num_sms, cudaStream_t s);
+// Filtered rows Y (nc apart) of views [v0, v0 + nv) -> row pairs of the stack `out`; vscale: FP16.
+void launch_row_pairs(const float *Y, int v0, int nv, int nc, bool centred, const float *vscale, void *out,
+                      int num_sms, cudaStream_t s);
+
 // How a block writes its sums: overwrite, add (views processed in order by successive launches)
 // or add atomically (several blocks of one launch share the voxels; the volume starts at zero).
 enum BpMode : int { kBpStore = 0, kBpAccumulate = 1, kBpAtomic = 2 };
@@ -134,13 +142,18 @@ inline bool queue_zpt_ok(int zpt) { return zpt == 1 || zpt == 4 || zpt == 8 || z
 // one voxel per thread along z (2D images; needs many resident warps to hide its gather latency),
 // class 1 tiles of 4, 8 or 16 (volumes; needs registers for its accumulators), class 2 the tiles
 // of quarter-turn items (BpArgs.sym set, interleaved partner stacks): first-quadrant columns,
-// 8 voxels per thread along z (1 for 2D images), view ranges counted in base views.
-constexpr int kQueueClasses = 3;
-constexpr int kQueueSymClass = 2;
+// 8 voxels per thread along z (1 for 2D images), view ranges counted in base views; class 3 planar items
+// over row pairs.
+constexpr int kQueueClasses = 4;
+constexpr int kQueueSymClass = 2, kQueueRowsClass = 3;
+constexpr int kRowsTileX = 64, kRowsTileY = 32;  // pixels of a planar tile: two cells, 8 pixels per thread
 inline bool sym_queue_zpt_ok(int zpt) { return zpt == 1 || zpt == 8; }
 inline int queue_class(int zpt) { return zpt == 1 ? 0 : 1; }
 // Blocks of a queue kernel resident per SM for the storage type (0 f32, 1 f16) and depth class.
 int queue_blocks_per_sm(int storage, int zclass);
+int rows_queue_blocks_per_sm(int storage);
+void launch_rows_queue(const BpItem *items, const BpWork *work, int n_work, int *counter, int storage, int grid,
+                       cudaStream_t s);
 // Launches grid blocks that take work entries [0, n_work) in order from *counter (zeroed by the
 // caller before the launch) until none are left. Every entry's item must be of the depth class.
 void launch_backproject_queue(const BpItem *items, const BpWork *work, int n_work, int *counter, int storage,

@@ -95,10 +95,9 @@ struct gct_fdk_plan {
     int nv = 0, nr = 0, nc = 0;
     float l1 = 0.f;
     int zpt = 8, bx = 32, by = 8;
-    // One-row 1D parallel detectors run transposed (kT1dPitch): the backprojector sees the image
-    // as kx x 1 x kz voxels (z = image y) over a one-column detector of nc rows.
-    bool t1d = false;
-    int kx = 0, ky = 0, kz = 0;  // backprojector grid (the image's [z][y][x] memory either way)
+    // Planar kinds whose filtered stack is row pairs with a backprojector of its own (rows.cu)
+    bool rows = false;
+    int kx = 0, ky = 0, kz = 0;  // backprojector grid
     // Quarter-turn symmetry (+1 / -1 / 0, quarter_turn_symmetry): whole-scan backprojections then
     // run over the first quarter of the views and of the (x, y) columns, each thread serving the
     // four rotated columns from the four partner views, with zpt_sym voxels along z.
@@ -151,18 +150,26 @@ struct gct_fdk_plan {
     }
 
     size_t quad_bytes() const { return opts.storage == GCT_STORAGE_F16 ? 8 : 16; }
-    // Workspace layout: the quads of view v at v * view_bytes(), then (FP16 storage) the per-view
-    // maxima, scales and inverse scales, nv floats each, from quad_region() on.
+    // Workspace layout: the quads or row pairs of view v at v * view_stride(), then (FP16 storage) the
+    // per-view maxima, scales and inverse scales, nv floats each, from quad_region() on.
     size_t view_bytes() const
     {
         return static_cast<size_t>(nr + 2 * gct::kQuadPad) * (nc + 2 * gct::kQuadPad) * quad_bytes();
     }
-    size_t quad_region() const { return (static_cast<size_t>(nv) * view_bytes() + 255) & ~static_cast<size_t>(255); }
+    // Bytes between the views of a stack: row pairs take a part of view_bytes(), which budgets and the
+    // published workspace size keep counting with.
+    size_t view_stride() const
+    {
+        return rows ? static_cast<size_t>(nc + 2 * gct::kQuadPad) * (quad_bytes() / 2) : view_bytes();
+    }
+    static size_t round_up(size_t bytes) { return (bytes + 255) & ~static_cast<size_t>(255); }
+    size_t quad_region() const { return round_up(static_cast<size_t>(nv) * view_stride()); }
     size_t scale_bytes() const { return opts.storage == GCT_STORAGE_F16 ? 3 * sizeof(float) * nv : 0; }
-    size_t workspace_bytes() const { return quad_region() + scale_bytes(); }
+    size_t stack_bytes() const { return quad_region() + scale_bytes(); }
+    size_t workspace_bytes() const { return round_up(static_cast<size_t>(nv) * view_bytes()) + scale_bytes(); }
 };
 
-// One filtered stack: the quads of view v at quads + v * view_bytes() and, for FP16 storage, the
+// One filtered stack: the quads or row pairs of view v at quads + v * view_stride() and, for FP16 storage, the
 // view's maximum, scale and inverse scale at amax[v], vscale[v], vinv[v]. All four are view-0
 // addresses, so a chunk of views may live at a shifted base.
 struct StackRef {
@@ -178,7 +185,7 @@ inline StackRef stack_of(const gct_fdk_plan *p, void *workspace, bool view_major
 {
     StackRef r;
     r.quads = static_cast<unsigned char *>(workspace);
-    r.quarter = (p->sym && !view_major) ? p->nv / 4 : 0;
+    r.quarter = (p->sym && !p->rows && !view_major) ? p->nv / 4 : 0;
     if (p->opts.storage == GCT_STORAGE_F16) {
         r.amax = reinterpret_cast<float *>(r.quads + p->quad_region());
         r.vscale = r.amax + p->nv;

@@ -1,0 +1,439 @@
+// Backprojection of one-row detectors (1D parallel, fan line, fan arc) into 2D images.
+//
+// A filtered view is one row of sample pairs (row pairs, kernels.hpp): a sample is one 8-byte (FP16
+// storage: 4-byte) load and one FMA, where a quad of a one-row view is 16 bytes (8) of which half hold
+// zeros. The image is cut into cells of 32 x 32 pixels; 128 threads own a cell, eight pixels each
+// along y, and keep the sums in registers over the views. The lanes of a warp cover 8 x 4 pixels per
+// step, so that its gathers fall into one to three cache lines whatever the view's direction, and the
+// eight pixels of a thread share the x part of the view's forms and run in packed FP32x2 pairs.
+//
+// Coordinates are evaluated in the same FP32 steps as in the quad kernels (backproject.cu), and FP16
+// storage blends in half precision as they do: the rounding of a coordinate of 2000 samples is most of
+// an image's error, and it stays what it was.
+//
+// Bound by instruction issue: about 7 (parallel), 10 (line) and 17 (arc) instructions per update.
+// Filter and backprojection, against the quad kernels over one-row views: parallel 1024 x 1024, 900 views
+// of 1455: 1.81 -> 0.47 ms; arc 509 x 387, 1151 views of 671: 1.13 -> 0.28 ms; line 512 x 512, 720 views
+// of 768, FP16: 0.208 -> 0.161 ms.
+// Cells per image are few (1024^2: 1024), so the views of a cell are cut into up to eight chunks, one
+// per block of a thread-block cluster; the blocks sum their parts through distributed shared memory
+// in chunk order and each writes its share of the cell, so there are no partial images and the
+// result does not depend on timing.
+#include <cooperative_groups.h>
+#include <cuda_runtime.h>
+
+#include "../../include/gct_fdk.h"
+#include "common.cuh"
+#include "geometry.hpp"
+#include "kernels.hpp"
+
+namespace gct {
+namespace {
+
+namespace cg = cooperative_groups;
+
+constexpr int kCell = 32;              // cell side in pixels
+constexpr int kThreads = 128;          // threads per cell: four warps side by side along x
+constexpr int kPairs = 4;              // pixel pairs per thread: pixels 4 apart along y
+constexpr int kStage = 32;             // views staged per barrier
+constexpr float kShift = 12582912.0f;  // 1.5 * 2^23: a sum with it holds a whole number in its low bits
+constexpr unsigned kShiftBits = 0x4B400000u;
+
+// One view of a cell: a = first form (u, U or A) at pixel (0, 0), per i and j step, and the weight
+// scale; b = second form (D or B) and 1 / dgamma; c0 = column of an arc's central ray.
+struct CellView {
+    float4 a, b;
+    float c0;
+    int cls;
+};
+constexpr int kOff = 0, kInside = 1, kMixed = 2;  // the cell projects off the row, well inside it, or neither
+
+// Where the thread's pixels are evaluated: at themselves, or in quarter-turn plans under the turns
+// that take the view to its base view. var: the index that varies over the thread's pixels (j; the
+// base view's i after an odd number of turns), c: the other one. Parallel kind: var counts from the
+// rows j0 and j0 + 16 of the cell (pairs 0, 1 and 2, 3).
+struct Pixels {
+    float2 var[kPairs];
+    float c, k0;
+};
+
+__device__ __forceinline__ float2 two(float x) { return make_float2(x, x); }
+
+// A form at the thread's pixel pair p, in the quad kernels' order: c0 + ci i, then + cj j.
+template <bool ODD>
+__device__ __forceinline__ float2 form(float4 f, const Pixels &px, int p)
+{
+    if (ODD) return __ffma2_rn(two(f.z), two(px.c), __ffma2_rn(two(f.y), px.var[p], two(f.x)));
+    return __ffma2_rn(two(f.z), px.var[p], two(fmaf(f.y, px.c, f.x)));
+}
+
+// Two samples at byte offsets o0, o1. Line and arc kinds: (y, dy) at column fractions f in [0, 1];
+// FP16 blends in half precision. Parallel kind (CENTRED): (mean, dy) at centred fractions, in FP32.
+struct RowF32 {
+    static constexpr unsigned kBytes = 8;
+    template <bool CENTRED>
+    static __device__ __forceinline__ float2 sample(const char *row, unsigned o0, unsigned o1, float2 f)
+    {
+        const float2 e0 = __ldg(reinterpret_cast<const float2 *>(row + o0));
+        const float2 e1 = __ldg(reinterpret_cast<const float2 *>(row + o1));
+        return make_float2(fmaf(f.x, e0.y, e0.x), fmaf(f.y, e1.y, e1.x));
+    }
+};
+struct RowF16 {
+    static constexpr unsigned kBytes = 4;
+    template <bool CENTRED>
+    static __device__ __forceinline__ float2 sample(const char *row, unsigned o0, unsigned o1, float2 f)
+    {
+        const __half2 h0 = __ldg(reinterpret_cast<const __half2 *>(row + o0));
+        const __half2 h1 = __ldg(reinterpret_cast<const __half2 *>(row + o1));
+        if (CENTRED) {
+            const float2 e0 = __half22float2(h0), e1 = __half22float2(h1);
+            return make_float2(fmaf(f.x, e0.y, e0.x), fmaf(f.y, e1.y, e1.x));
+        }
+        return __half22float2(__hfma2(__floats2half2_rn(f.x, f.y), __highs2half2(h0, h1), __lows2half2(h0, h1)));
+    }
+};
+
+// Adds one view to the thread's pixels. INSIDE: the cell's samples lie well inside the row (and in
+// front of an arc's source, near its axis); else pixels that project off the row add nothing.
+template <int FAMILY, class R, bool ODD, bool INSIDE>
+__device__ __forceinline__ void add_view(const CellView &v, const char *row, float umax, const Pixels &px,
+                                         float2 (&acc)[kPairs])
+{
+    const float4 a = v.a, b = v.b;
+    float v0[2] = {0.f, 0.f};
+    if (FAMILY == 0) {  // rows j0 and j0 + 16, less the half of the centred split
+        const float u = fmaf(a.y, px.c, a.x);
+        v0[0] = fmaf(a.z, px.k0, u) - 0.5f;
+        v0[1] = fmaf(a.z, px.k0 + 16.f, u) - 0.5f;
+    }
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) {
+        float2 u, w = two(a.w), t;
+        if (FAMILY == 0) {
+            u = __ffma2_rn(two(a.z), px.var[p], two(v0[p / 2]));
+            if (!INSIDE)  // where the row's zero border is
+                u = make_float2(fminf(fmaxf(u.x, -1.5f), umax - 0.5f), fminf(fmaxf(u.y, -1.5f), umax - 0.5f));
+            t = __fadd2_rn(u, two(kShift));
+        } else {
+            u = form<ODD>(a, px, p);
+            const float2 d = form<ODD>(b, px, p);
+            if (FAMILY == 1) {
+                const float2 inv = make_float2(rcp_approx(d.x), rcp_approx(d.y));
+                u = __fmul2_rn(u, inv);
+                w = __fmul2_rn(__fmul2_rn(w, inv), inv);
+            } else {
+                const float2 rho2 = __ffma2_rn(u, u, __fmul2_rn(d, d));
+                w = __fmul2_rn(w, make_float2(rcp_approx(rho2.x), rcp_approx(rho2.y)));
+                const float2 g = INSIDE ? arc_angle_near(u, d) : make_float2(atan2f(u.x, d.x), atan2f(u.y, d.y));
+                u = __ffma2_rn(g, two(b.w), two(v.c0));
+            }
+        }
+        bool on0 = true, on1 = true;
+        if (FAMILY != 0) {
+            if (!INSIDE) {
+                on0 = u.x >= -1.0f && u.x <= umax;
+                on1 = u.y >= -1.0f && u.y <= umax;
+                u = make_float2(on0 ? u.x : -1.0f, on1 ? u.y : -1.0f);
+            }
+            t = __fadd2_rd(u, two(kShift));  // floor
+        }
+        const float2 f = __ffma2_rn(__fadd2_rn(t, two(-kShift)), two(-1.f), u);
+        constexpr unsigned kBase = (static_cast<unsigned>(kQuadPad) - kShiftBits) * R::kBytes;  // modulo 2^32
+        const float2 val = R::template sample<FAMILY == 0>(row, __float_as_uint(t.x) * R::kBytes + kBase,
+                                                           __float_as_uint(t.y) * R::kBytes + kBase, f);
+        const float2 r = __ffma2_rn(w, val, acc[p]);
+        if (on0) acc[p].x = r.x;
+        if (on1) acc[p].y = r.y;
+    }
+}
+
+// Index box of a cell's pixels in the image.
+struct Box {
+    float i0, i1, j0, j1;
+};
+
+// Stages view v (base view b, its pixels in box) for the cell and classifies it: the coordinate is
+// linear, or linear-fractional with a positive denominator (arc: its tangent), so that its extremes
+// are at the corners; 1/64 of a sample covers the rounding.
+template <int FAMILY>
+__device__ void stage_view(const BpArgs &a, int v, int b, const Box &box, CellView &out)
+{
+    const float *c = a.coefs + static_cast<long long>(b) * kCoefPerView;
+    constexpr int kD = FAMILY == 1 ? 8 : 4, kW = FAMILY == 0 ? 5 : FAMILY == 1 ? 12 : 16;
+    float w = __ldg(a.coefs + static_cast<long long>(v) * kCoefPerView + kW);
+    if (a.vinv) w *= __ldg(a.vinv + v);
+    out.a = make_float4(__ldg(c), __ldg(c + 1), __ldg(c + 2), w);
+    out.b = FAMILY == 0 ? make_float4(0.f, 0.f, 0.f, 0.f)
+                        : make_float4(__ldg(c + kD), __ldg(c + kD + 1), __ldg(c + kD + 2), __ldg(c + 12));
+    out.c0 = FAMILY == 2 ? __ldg(c + 13) : 0.f;
+    float lo = 3.0e38f, hi = -3.0e38f;
+    bool plain = true;
+#pragma unroll
+    for (int k = 0; k < 4; ++k) {
+        const float i = (k & 1) ? box.i1 : box.i0, j = (k & 2) ? box.j1 : box.j0;
+        float u = fmaf(out.a.z, j, fmaf(out.a.y, i, out.a.x));
+        if (FAMILY != 0) {
+            const float d = fmaf(out.b.z, j, fmaf(out.b.y, i, out.b.x));
+            if (!(d > 0.f) || (FAMILY == 2 && !(fabsf(u) <= kArcNear * d))) plain = false;
+            u = FAMILY == 1 ? u / d : fmaf(atan2f(u, d), out.b.w, out.c0);
+        }
+        lo = fminf(lo, u);
+        hi = fmaxf(hi, u);
+    }
+    const float m = 1.0f / 64.0f;
+    out.cls = !plain                                   ? kMixed
+              : hi < -1.0f - m || lo > a.umax + m      ? kOff
+              : lo >= -1.0f + m && hi <= a.umax - m    ? kInside
+                                                       : kMixed;
+}
+
+// Sums of views [a.v_begin, a.v_begin + a.v_count) for the 128 threads of the cell at pixel (i0, j0);
+// every thread of the block calls it (it holds block barriers), tid counts within the cell. SYM:
+// quarter-turn plans, whose views take their coordinates from the base view at the turned pixel.
+template <int FAMILY, class R, bool SYM>
+__device__ __forceinline__ void cell_sums(const BpArgs &a, int i0, int j0, int tid, CellView *s_view,
+                                          float2 (&acc)[kPairs])
+{
+    const int lane = tid & 31;
+    // pixels past the image's last ones repeat them (samples have to lie where the cell's class says)
+    // and are not stored
+    const float i1 = static_cast<float>(max(min(i0 + kCell, a.nx) - 1, i0));
+    const float j1 = static_cast<float>(max(min(j0 + kCell, a.ny) - 1, j0));
+    const float fi = fminf(static_cast<float>(i0 + (tid >> 5) * 8 + (lane & 7)), i1);
+    const float fj = static_cast<float>(j0 + (lane >> 3));
+    Pixels px;
+    px.c = fi;
+    px.k0 = static_cast<float>(j0);
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) {
+        acc[p] = make_float2(0.f, 0.f);
+        px.var[p] = make_float2(fminf(fj + 8.f * p, j1), fminf(fj + 8.f * p + 4.f, j1));
+        if (FAMILY == 0) {
+            const float k = px.k0 + 16.f * (p / 2);
+            px.var[p] = make_float2(px.var[p].x - k, px.var[p].y - k);
+        }
+    }
+    const int row_bytes = (static_cast<int>(a.qview)) * static_cast<int>(R::kBytes);
+    int v = a.v_begin;
+    const int end = a.v_begin + a.v_count;
+    while (v < end) {
+        // views [v, stop) of one quarter: q turns from their base views
+        const int q = SYM ? v / a.quarter : 0, stop = SYM ? min(end, (q + 1) * a.quarter) : end;
+        Box box{static_cast<float>(i0), i1, static_cast<float>(j0), j1};
+        if (SYM) {
+            // R^-q of (i, j): (n-1-i, n-1-j) after two turns, (j, n-1-i) or (n-1-j, i) after one or three
+            const float n1 = static_cast<float>(a.nx - 1);
+            const bool flip_j = q == 2 || q == (a.sym > 0 ? 3 : 1), flip_i = q == 2 || q == (a.sym > 0 ? 1 : 3);
+            px.c = flip_i ? n1 - fi : fi;
+#pragma unroll
+            for (int p = 0; p < kPairs; ++p) {
+                const float y0 = fminf(fj + 8.f * p, j1), y1 = fminf(fj + 8.f * p + 4.f, j1);
+                px.var[p] = flip_j ? make_float2(n1 - y0, n1 - y1) : make_float2(y0, y1);
+            }
+            if (flip_i) box.i0 = n1 - i1, box.i1 = n1 - static_cast<float>(i0);
+            if (flip_j) box.j0 = n1 - j1, box.j1 = n1 - static_cast<float>(j0);
+            if (q & 1) box = Box{box.j0, box.j1, box.i0, box.i1};
+        }
+        for (; v < stop; v += kStage) {
+            const int nvc = min(kStage, stop - v);
+            __syncthreads();
+            if (tid < nvc) stage_view<FAMILY>(a, v + tid, v + tid - q * (SYM ? a.quarter : 0), box, s_view[tid]);
+            __syncthreads();
+            const char *row = static_cast<const char *>(a.quads) + static_cast<long long>(v) * row_bytes;
+            for (int k = 0; k < nvc; ++k, row += row_bytes) {
+                const int cls = s_view[k].cls;
+                if (cls == kOff) continue;  // every pixel of the cell would add zero
+                if (SYM && (q & 1)) {
+                    if (cls == kInside) add_view<FAMILY, R, true, true>(s_view[k], row, a.umax, px, acc);
+                    else add_view<FAMILY, R, true, false>(s_view[k], row, a.umax, px, acc);
+                } else {
+                    if (cls == kInside) add_view<FAMILY, R, false, true>(s_view[k], row, a.umax, px, acc);
+                    else add_view<FAMILY, R, false, false>(s_view[k], row, a.umax, px, acc);
+                }
+            }
+        }
+        v = stop;
+    }
+}
+
+// A cluster of gridDim.z blocks per cell, each with its chunk of the views.
+template <int FAMILY, class R, bool SYM>
+__global__ void __launch_bounds__(kThreads, 8) rows_kernel(BpArgs a, int chunk)
+{
+    __shared__ CellView s_view[kStage];
+    __shared__ float s_sum[kCell * kCell];  // [pixel][thread]: the block's sums
+    const int i0 = blockIdx.x * kCell, j0 = blockIdx.y * kCell, tid = threadIdx.x;
+    const int z = blockIdx.z, chunks = gridDim.z;
+    BpArgs la = a;
+    la.v_begin = a.v_begin + z * chunk;
+    la.v_count = max(0, min(chunk, a.v_count - z * chunk));
+    float2 acc[kPairs];
+    cell_sums<FAMILY, R, SYM>(la, i0, j0, tid, s_view, acc);
+    const int i = i0 + (tid >> 5) * 8 + (tid & 7), j = j0 + ((tid >> 3) & 3);
+    auto put = [&](int p, float s) {
+        const int y = j + 4 * p;
+        if (i >= a.nx || y >= a.ny) return;
+        float *dst = a.vol + static_cast<long long>(y) * a.nx + i;
+        *dst = a.accumulate ? *dst + s : s;
+    };
+    if (chunks == 1) {
+#pragma unroll
+        for (int p = 0; p < 2 * kPairs; ++p) put(p, (p & 1) ? acc[p / 2].y : acc[p / 2].x);
+        return;
+    }
+#pragma unroll
+    for (int p = 0; p < 2 * kPairs; ++p) s_sum[p * kThreads + tid] = (p & 1) ? acc[p / 2].y : acc[p / 2].x;
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();
+    // the block's share of the pixels (the chunks are 2, 4 or 8), over the chunks in order
+    for (int p = z; p < 2 * kPairs; p += chunks) {
+        float s = 0.f;
+        for (int c = 0; c < chunks; ++c) s += cl.map_shared_rank(s_sum, c)[p * kThreads + tid];
+        put(p, s);
+    }
+    cl.sync();  // the sums stay until every block has read them
+}
+
+// Work-queue form: 256 threads take a tile of two cells side by side.
+template <int FAMILY, class R, bool SYM>
+__device__ __noinline__ void queue_cells(const BpArgs &a, int tx, int ty, int tid, int mode, CellView *s_view)
+{
+    const int i0 = (2 * tx + tid / kThreads) * kCell, j0 = ty * kCell, ct = tid % kThreads;
+    float2 acc[kPairs];
+    cell_sums<FAMILY, R, SYM>(a, i0, j0, ct, s_view + (tid / kThreads) * kStage, acc);
+    const int i = i0 + (ct >> 5) * 8 + (ct & 7), j = j0 + ((ct >> 3) & 3);
+#pragma unroll
+    for (int p = 0; p < 2 * kPairs; ++p) {
+        const int y = j + 4 * p;
+        if (i >= a.nx || y >= a.ny) continue;
+        const float s = (p & 1) ? acc[p / 2].y : acc[p / 2].x;
+        float *dst = a.vol + static_cast<long long>(y) * a.nx + i;
+        if (mode == kBpAtomic) atomicAdd(dst, s);
+        else *dst = mode == kBpAccumulate ? *dst + s : s;
+    }
+}
+
+template <class R>
+__global__ void __launch_bounds__(kQueueThreads, 4)
+    rows_queue_kernel(const BpItem *__restrict__ items, const BpWork *__restrict__ work, int n_work, int *counter)
+{
+    static_assert(kRowsTileX == (kQueueThreads / kThreads) * kCell && kRowsTileY == kCell, "tile of two cells");
+    __shared__ CellView s_view[kQueueThreads / kThreads * kStage];
+    __shared__ BpItem s_item;
+    __shared__ BpWork s_work;
+    __shared__ int s_next;
+    const int tid = threadIdx.x;
+    for (;;) {
+        if (tid == 0) s_next = atomicAdd(counter, 1);
+        __syncthreads();
+        const int w = s_next;
+        if (w >= n_work) return;
+        if (tid == 0) {
+            s_work = work[w];
+            s_item = items[s_work.item];
+        }
+        __syncthreads();
+        BpArgs a = s_item.a;
+        a.v_begin = s_work.v_begin;
+        a.v_count = s_work.v_count;
+        const int mode = s_work.mode, tx = s_work.tile % s_item.tiles_x, ty = s_work.tile / s_item.tiles_x;
+        if (s_item.family == 0) {
+            queue_cells<0, R, false>(a, tx, ty, tid, mode, s_view);
+        } else if (s_item.family == 1) {
+            if (a.sym) queue_cells<1, R, true>(a, tx, ty, tid, mode, s_view);
+            else queue_cells<1, R, false>(a, tx, ty, tid, mode, s_view);
+        } else if constexpr (R::kBytes == RowF32::kBytes) {  // FP16 arcs keep their quads
+            if (a.sym) queue_cells<2, R, true>(a, tx, ty, tid, mode, s_view);
+            else queue_cells<2, R, false>(a, tx, ty, tid, mode, s_view);
+        }
+        __syncthreads();  // s_item / s_work / s_next are rewritten for the next entry
+    }
+}
+
+// Filtered rows Y (row stride nc, views v0 on) -> row pairs.
+template <bool F16>
+__global__ void row_pairs_kernel(const float *__restrict__ Y, int v0, int nv, int nc, bool centred,
+                                 const float *__restrict__ vscale, void *out)
+{
+    const int pitch = nc + 2 * kQuadPad;
+    const long long n = static_cast<long long>(nv) * pitch;
+    for (long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
+         e += static_cast<long long>(gridDim.x) * blockDim.x) {
+        const int v = static_cast<int>(e / pitch), c = static_cast<int>(e - static_cast<long long>(v) * pitch) - kQuadPad;
+        const float *y = Y + static_cast<long long>(v) * nc;
+        const float sc = F16 ? __ldg(vscale + v0 + v) : 1.f;
+        const float y0 = c >= 0 && c < nc ? sc * __ldg(y + c) : 0.f;
+        const float y1 = c + 1 >= 0 && c + 1 < nc ? sc * __ldg(y + c + 1) : 0.f;
+        store_row_pair<F16>(out, static_cast<long long>(v0) * pitch + e, y0, y1, centred);
+    }
+}
+
+template <class R>
+void launch_rows(const BpArgs &a, int family, int num_sms, cudaStream_t s)
+{
+    const dim3 cells((a.nx + kCell - 1) / kCell, (a.ny + kCell - 1) / kCell);
+    // chunks of at least 8 views until the grid holds six waves of eight blocks per SM: the last wave
+    // of a launch of one to two waves runs nearly empty
+    const long long want = 6LL * 8 * num_sms;
+    int chunks = 1;
+    while (chunks < 8 && static_cast<long long>(cells.x) * cells.y * chunks < want && a.v_count / (2 * chunks) >= 8)
+        chunks *= 2;
+    const int chunk = (a.v_count + chunks - 1) / chunks;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(cells.x, cells.y, chunks);
+    cfg.blockDim = dim3(kThreads);
+    cfg.stream = s;
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeClusterDimension;
+    at[0].val.clusterDim.x = 1;
+    at[0].val.clusterDim.y = 1;
+    at[0].val.clusterDim.z = static_cast<unsigned>(chunks);
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    if (family == 0) {
+        cudaLaunchKernelEx(&cfg, rows_kernel<0, R, false>, a, chunk);
+    } else if (family == 1) {
+        if (a.sym) cudaLaunchKernelEx(&cfg, rows_kernel<1, R, true>, a, chunk);
+        else cudaLaunchKernelEx(&cfg, rows_kernel<1, R, false>, a, chunk);
+    } else if constexpr (R::kBytes == RowF32::kBytes) {
+        if (a.sym) cudaLaunchKernelEx(&cfg, rows_kernel<2, R, true>, a, chunk);
+        else cudaLaunchKernelEx(&cfg, rows_kernel<2, R, false>, a, chunk);
+    }
+}
+
+}  // namespace
+
+void launch_backproject_rows(const BpArgs &a, int family, int storage, int num_sms, cudaStream_t s)
+{
+    if (storage == 0) launch_rows<RowF32>(a, family, num_sms, s);
+    else launch_rows<RowF16>(a, family, num_sms, s);
+}
+
+int rows_queue_blocks_per_sm(int storage)
+{
+    int n = 0;
+    const cudaError_t e =
+        storage == 0 ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rows_queue_kernel<RowF32>, kQueueThreads, 0)
+                     : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&n, rows_queue_kernel<RowF16>, kQueueThreads, 0);
+    return e == cudaSuccess ? n : 0;
+}
+
+void launch_rows_queue(const BpItem *items, const BpWork *work, int n_work, int *counter, int storage, int grid,
+                       cudaStream_t s)
+{
+    if (storage == 0) rows_queue_kernel<RowF32><<<grid, kQueueThreads, 0, s>>>(items, work, n_work, counter);
+    else rows_queue_kernel<RowF16><<<grid, kQueueThreads, 0, s>>>(items, work, n_work, counter);
+}
+
+void launch_row_pairs(const float *Y, int v0, int nv, int nc, bool centred, const float *vscale, void *out,
+                      int num_sms, cudaStream_t s)
+{
+    long long grid = (static_cast<long long>(nv) * (nc + 2 * kQuadPad) + 255) / 256;
+    if (grid > static_cast<long long>(num_sms) * 32) grid = static_cast<long long>(num_sms) * 32;
+    const unsigned g = static_cast<unsigned>(grid < 1 ? 1 : grid);
+    if (vscale) row_pairs_kernel<true><<<g, 256, 0, s>>>(Y, v0, nv, nc, centred, vscale, out);
+    else row_pairs_kernel<false><<<g, 256, 0, s>>>(Y, v0, nv, nc, centred, vscale, out);
+}
+
+}  // namespace gct

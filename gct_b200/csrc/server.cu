@@ -233,7 +233,7 @@ void run_round(gct_fdk_server *s)
     std::vector<std::pair<Request *, int>> advanced;
     for (Request *r : s->active) {
         const int q = (r->plan->opts.storage == GCT_STORAGE_F16 ? 1 : 0) * gct::kQueueClasses +
-                      gct::item_class(r->st, r->cfg);
+                      gct::item_class(r->plan, r->st, r->cfg);
         const int vb = r->next_view, vc = std::min(r->chunk, gct::item_views(r->plan, r->st) - vb);
         const gct::BpItem it = gct::make_item(r->plan, r->st, r->vol_dev, r->cfg);
         const int idx = static_cast<int>(items[q].size());
