@@ -268,11 +268,13 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
     if (p->sym && !p->rows && !p->ybuf.p)
         p->ybuf.alloc(static_cast<size_t>(p->nv) * p->nr * p->nc, "filtered rows of quarter-turn stacks");
     if (p->spiral) {
-        // one slice per thread along z: each slice has its own window of views
+        // each slice has its own window of views: z-affine geometries take several slices per thread
+        // over the union of their windows, others one
         p->sym = 0;
-        p->zpt = 1;
-        if (p->opts.block_x <= 0) p->bx = 32;
-        if (p->opts.block_y <= 0) p->by = 8;
+        if (p->opts.z_per_thread <= 0) p->zpt = 8;
+        if (!p->z_affine || p->zpt < 4) p->zpt = 1;
+        if (p->opts.block_x <= 0) p->bx = f16 ? 8 : 4;
+        if (p->opts.block_y <= 0) p->by = 16;
         std::vector<int2> win(p->kz);
         const double z0 = vol->mid[2] - (vol->nz - 1.0) * vol->dz / 2.0;
         for (int k = 0; k < p->kz; ++k) {
