@@ -74,9 +74,11 @@ template <class Q> struct LerpOf;
 template <> struct LerpOf<QuadF32> { using type = LerpF32; };
 template <> struct LerpOf<QuadF16> { using type = LerpF16; };
 
+// Weights of a voxel or of the voxel pair (z, z + 1), element for element the same roundings.
 struct ConstWeight {
     float w;
     __device__ __forceinline__ float at(int) const { return w; }
+    __device__ __forceinline__ float2 at2(int) const { return make_float2(w, w); }
 };
 struct ArcWeight {  // wscale / (rho^2 + T(z)^2), T(z) = T0 + z tk
     float ws, rho2, T0, tk;
@@ -84,6 +86,13 @@ struct ArcWeight {  // wscale / (rho^2 + T(z)^2), T(z) = T0 + z tk
     {
         const float T = fmaf(tk, static_cast<float>(z), T0);
         return ws * rcp_approx(fmaf(T, T, rho2));
+    }
+    __device__ __forceinline__ float2 at2(int z) const
+    {
+        const float2 T = __ffma2_rn(make_float2(tk, tk), make_float2(static_cast<float>(z), static_cast<float>(z + 1)),
+                                    make_float2(T0, T0));
+        const float2 r = __ffma2_rn(T, T, make_float2(rho2, rho2));
+        return __fmul2_rn(make_float2(ws, ws), make_float2(rcp_approx(r.x), rcp_approx(r.y)));
     }
 };
 
@@ -131,7 +140,7 @@ __device__ __forceinline__ void column(unsigned long long base, int stride, type
             const auto *p1 = reinterpret_cast<const typename L::S *>(
                 base + static_cast<unsigned long long>(static_cast<long long>(__float_as_int(t.y)) * stride));
             const float2 val = make_float2(L::lerp(__ldg(p0), fu, fvc.x), L::lerp(__ldg(p1), fu, fvc.y));
-            const float2 r = __ffma2_rn(make_float2(wt.at(z), wt.at(z + 1)), val, make_float2(acc[z], acc[z + 1]));
+            const float2 r = __ffma2_rn(wt.at2(z), val, make_float2(acc[z], acc[z + 1]));
             if (!SOME || ((on >> z) & 1u)) acc[z] = r.x;
             if (!SOME || ((on >> z) & 2u)) acc[z + 1] = r.y;
             if constexpr (MIRROR) {
@@ -153,7 +162,7 @@ __device__ __forceinline__ void column(unsigned long long base, int stride, type
                     valm = make_float2(L::lerp(__ldg(q0), fu, -fvc.x), L::lerp(__ldg(q1), fu, -fvc.y));
                 }
                 float(&dm)[ZPT] = *accm;
-                const float2 rm = __ffma2_rn(make_float2(wt.at(z), wt.at(z + 1)), valm, make_float2(dm[z], dm[z + 1]));
+                const float2 rm = __ffma2_rn(wt.at2(z), valm, make_float2(dm[z], dm[z + 1]));
                 dm[z] = rm.x;
                 dm[z + 1] = rm.y;
             }
@@ -602,6 +611,8 @@ void launch_q(const BpArgs &a, bool z_affine, int zpt, int bx, int by, cudaStrea
 struct ConstWeight4 {
     float w[4];
     __device__ __forceinline__ float at(int q, int) const { return w[q]; }
+    __device__ __forceinline__ float2 common(int) const { return make_float2(1.f, 1.f); }
+    __device__ __forceinline__ float2 at2(int q, float2) const { return make_float2(w[q], w[q]); }
 };
 struct ArcWeight4 {
     float ws[4];
@@ -611,6 +622,15 @@ struct ArcWeight4 {
         const float T = fmaf(tk, static_cast<float>(z), T0);
         return ws[q] * rcp_approx(fmaf(T, T, rho2));
     }
+    // of the voxel pair (z, z + 1): the factor common to the partners, then partner q's weights
+    __device__ __forceinline__ float2 common(int z) const
+    {
+        const float2 T = __ffma2_rn(make_float2(tk, tk), make_float2(static_cast<float>(z), static_cast<float>(z + 1)),
+                                    make_float2(T0, T0));
+        const float2 r = __ffma2_rn(T, T, make_float2(rho2, rho2));
+        return make_float2(rcp_approx(r.x), rcp_approx(r.y));
+    }
+    __device__ __forceinline__ float2 at2(int q, float2 c) const { return __fmul2_rn(make_float2(ws[q], ws[q]), c); }
 };
 
 // The four partner quads of one detector position in the quarter-turn layout (quad_layout): 32
@@ -656,11 +676,12 @@ __device__ __forceinline__ void column4(unsigned long long base, int stride, typ
             typename L::S q0[4], q1[4];
             ldg_partners(base + static_cast<unsigned long long>(static_cast<long long>(__float_as_int(t.x)) * stride), q0);
             ldg_partners(base + static_cast<unsigned long long>(static_cast<long long>(__float_as_int(t.y)) * stride), q1);
+            const float2 wz = wt.common(z);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
                 const float2 val = make_float2(L::lerp(q0[q], fu, fvc.x), L::lerp(q1[q], fu, fvc.y));
                 float(&dst)[ZPT] = acc[(K + q) & 3];
-                const float2 r = __ffma2_rn(make_float2(wt.at(q, z), wt.at(q, z + 1)), val, make_float2(dst[z], dst[z + 1]));
+                const float2 r = __ffma2_rn(wt.at2(q, wz), val, make_float2(dst[z], dst[z + 1]));
                 dst[z] = r.x;
                 dst[z + 1] = r.y;
             }
