@@ -162,13 +162,8 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
     gct::SpiralInfo spiral_si;
     if (p->spiral) spiral_si = gct::spiral_info(p->geom);  // validates like SpiralCTGeom
     // spiral scans: no Parker weights (fdk_spiral.cuh applies cosine weights and the filter only)
-    std::vector<float> parker;
-    if (p->spiral) {
-        parker.assign(static_cast<size_t>(p->nv) * p->nc, 1.0f);
-    } else {
-        const std::vector<double> parker_d = gct::parker_table(p->geom, p->rot);
-        parker.assign(parker_d.begin(), parker_d.end());
-    }
+    gct::ParkerRule parker;
+    if (!p->spiral) parker = gct::parker_rule(p->geom, p->rot);
     const std::vector<double> taps = gct::ramp_taps(kind, g->det_row, p->filt);
     double l1 = 0.0;
     for (double t : taps) l1 += std::fabs(t);
@@ -179,16 +174,36 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
         H[k] = make_float2(static_cast<float>(Hd[k].real()), static_cast<float>(Hd[k].imag()));
 
     cuda_check(cudaGetDevice(&p->device), "cudaGetDevice");
-    cudaDeviceProp prop{};
-    cuda_check(cudaGetDeviceProperties(&prop, p->device), "cudaGetDeviceProperties");
-    p->num_sms = prop.multiProcessorCount;
-    p->fview.upload(fview.data(), fview.size(), "plan geometry");
-    p->parker.upload(parker.data(), parker.size(), "plan Parker table");
-    p->H.upload(H.data(), H.size(), "plan filter spectrum");
-    // status word of the plan's kernels (gct_fdk_plan_check): GEMM pipeline and FFT input waits
-    p->gemm_err.alloc(1, "kernel status");
-    cuda_check(cudaMemset(p->gemm_err.p, 0, sizeof(int)), "kernel status reset");
-    p->coefs.upload(coefs.data(), coefs.size(), "plan backprojection coefficients");
+    // (cudaGetDeviceProperties, which asks for everything, takes 2.6 ms)
+    cuda_check(cudaDeviceGetAttribute(&p->num_sms, cudaDevAttrMultiProcessorCount, p->device),
+               "cudaDeviceGetAttribute");
+    // the plan's tables in one allocation and one upload; the Parker table is computed in place
+    std::vector<unsigned char> blob;
+    auto put = [&blob](const void *src, size_t bytes) {
+        const size_t at = blob.size();
+        blob.resize(at + ((bytes + 255) & ~static_cast<size_t>(255)));
+        if (bytes) std::memcpy(blob.data() + at, src, bytes);
+        return at;
+    };
+    const int no_error = 0;  // status word of the plan's kernels (gct_fdk_plan_check)
+    const size_t at_err = put(&no_error, sizeof(int)), at_fview = put(fview.data(), fview.size() * sizeof(float4)),
+                 at_H = put(H.data(), H.size() * sizeof(float2)),
+                 at_coefs = put(coefs.data(), coefs.size() * sizeof(float)),
+                 at_gamma = put(parker.gamma.data(), parker.gamma.size() * sizeof(double)),
+                 at_rel = put(parker.rel.data(), parker.rel.size() * sizeof(double));
+    const size_t weights = static_cast<size_t>(p->nv) * p->nc;
+    p->tables.alloc(blob.size() + weights * sizeof(float), "plan tables");
+    cuda_check(cudaMemcpy(p->tables.p, blob.data(), blob.size(), cudaMemcpyHostToDevice), "plan tables");
+    p->gemm_err = reinterpret_cast<int *>(p->tables.p + at_err);
+    p->fview = reinterpret_cast<float4 *>(p->tables.p + at_fview);
+    p->H = reinterpret_cast<float2 *>(p->tables.p + at_H);
+    p->coefs = reinterpret_cast<float *>(p->tables.p + at_coefs);
+    p->parker = reinterpret_cast<float *>(p->tables.p + blob.size());
+    const double *gamma = parker.gamma.empty() ? nullptr : reinterpret_cast<double *>(p->tables.p + at_gamma);
+    gct::launch_parker(gamma, reinterpret_cast<double *>(p->tables.p + at_rel), parker.phi,
+                       static_cast<float>(parker.constant), p->nv, p->nc, p->parker, nullptr);
+    cuda_check(cudaGetLastError(), "Parker kernel launch");
+    cuda_check(cudaStreamSynchronize(nullptr), "plan tables");  // the plan may be used on any stream
     if (p->opts.filter != GCT_FILTER_FFT) {
         // B = T^T with T[k][c] = g(c - k): row n holds g(n - k); taps g(m) = taps[m + nc/2]
         p->Kp = gct::gemm_pad_k(p->nc);
@@ -306,8 +321,8 @@ void split_rows(gct_fdk_plan *p, const float *proj, int vb, int vc, int quarter,
     sa.kind = p->kind;
     sa.du = static_cast<float>(p->geom.det_row.sampling_width);
     sa.dv = static_cast<float>(p->geom.det_col.sampling_width);
-    sa.fview = p->fview.p;
-    sa.parker = p->parker.p;
+    sa.fview = p->fview;
+    sa.parker = p->parker;
     sa.xh = p->xh.p;
     sa.xl = p->xl.p;
     sa.xll = p->xll.p;
@@ -342,7 +357,7 @@ gct::GemmLaunch gemm_launch(const gct_fdk_plan *p)
     gl.Np = p->Np;
     gl.Kp = p->Kp;
     gl.N = p->nc;
-    gl.err = p->gemm_err.p;
+    gl.err = p->gemm_err;
     return gl;
 }
 
@@ -387,7 +402,7 @@ void run_filter_gemm(gct_fdk_plan *p, const float *proj, void *out, const float 
     qa.vscale = (mode == gct::kOutQuadF16) ? vscale : nullptr;
     qa.out = out;
     qa.quarter = quarter;
-    qa.err = p->gemm_err.p;
+    qa.err = p->gemm_err;
     gct::launch_quads_from_rows(qa, mode, p->num_sms, s);
     cuda_check(cudaGetLastError(), "quad kernel launch");
 }
@@ -414,10 +429,10 @@ void run_filter(gct_fdk_plan *p, const float *proj, void *out, const float *vsca
     fa.kind = p->kind;
     fa.du = static_cast<float>(p->geom.det_row.sampling_width);
     fa.dv = static_cast<float>(p->geom.det_col.sampling_width);
-    fa.fview = p->fview.p + vb;
-    fa.parker = p->parker.p + static_cast<long long>(vb) * p->nc;
-    fa.H = p->H.p;
-    fa.err = p->gemm_err.p;
+    fa.fview = p->fview + vb;
+    fa.parker = p->parker + static_cast<long long>(vb) * p->nc;
+    fa.H = p->H;
+    fa.err = p->gemm_err;
     fa.mode = mode;
     if (mode == gct::kOutPlainF32) {
         fa.out = static_cast<float *>(out) + vb * pix;
@@ -437,7 +452,7 @@ gct::BpArgs bp_args(const gct_fdk_plan *p, const StackRef &st, float *vol, int v
     ba.quads = st.quads;
     ba.qpitch = p->nc + 2 * gct::kQuadPad;
     ba.qview = static_cast<long long>(p->rows ? 1 : p->nr + 2 * gct::kQuadPad) * ba.qpitch;
-    ba.coefs = p->coefs.p;
+    ba.coefs = p->coefs;
     ba.vinv = st.vinv;
     ba.v_begin = v_begin;
     ba.v_count = v_count;
@@ -622,7 +637,7 @@ void prepare_partners(gct_fdk_plan *p, const float *proj, const StackRef &st, in
     qa.vscale = f16 ? st.vscale : nullptr;
     qa.out = st.quads;
     qa.quarter = m;
-    qa.err = p->gemm_err.p;
+    qa.err = p->gemm_err;
     gct::launch_quads_partners(qa, f16 ? gct::kOutQuadF16 : gct::kOutQuadF32, p->num_sms, s);
     cuda_check(cudaGetLastError(), "partner quad kernel launch");
 }
@@ -1059,11 +1074,11 @@ gct_status gct_fdk_plan_check(gct_fdk_plan *plan)
         if (!plan) gct::fail(GCT_ERR_INVALID_ARG, "NULL plan");
         DeviceGuard dg(plan->device);
         cuda_check(cudaDeviceSynchronize(), "device synchronisation");
-        if (!plan->gemm_err.p) return;
+        if (!plan->gemm_err) return;
         int e = 0;
-        cuda_check(cudaMemcpy(&e, plan->gemm_err.p, sizeof(int), cudaMemcpyDeviceToHost), "GEMM status read");
+        cuda_check(cudaMemcpy(&e, plan->gemm_err, sizeof(int), cudaMemcpyDeviceToHost), "GEMM status read");
         if (e) {
-            cuda_check(cudaMemset(plan->gemm_err.p, 0, sizeof(int)), "kernel status reset");
+            cuda_check(cudaMemset(plan->gemm_err, 0, sizeof(int)), "kernel status reset");
             if (e & gct::kFftWaitTimeout)
                 gct::fail(GCT_ERR_TIMEOUT, "FFT filter: a projection row copy did not arrive within 2 s");
             if (e & gct::kQuadWaitTimeout)
@@ -1239,24 +1254,29 @@ gct_status gct_reconstruct_ex(const gct_ct_geom *geom, const gct_vol_geom *vol,
         // reconFDK's choice (src/cuda/recon/fdk_axial.cuh:68-89): all projections on the device
         // when they, the volume and the filtered stack need under 75 % of the device memory,
         // else the streaming path with half of the memory left after the volume
-        size_t free_b = 0, total_b = 0;
-        cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
-        const double req = static_cast<double>(proj_n + vol_n) * sizeof(float) + static_cast<double>(p->workspace_bytes());
-        if (req >= 0.75 * static_cast<double>(total_b)) {
-            const size_t vol_b = vol_n * sizeof(float);
-            execute_host_budget(p, proj_host, vol_host, free_b > vol_b ? (free_b - vol_b) / 2 : 0, nullptr);
-            return;
+        const size_t vol_b = vol_n * sizeof(float);
+        const double req = static_cast<double>(proj_n) * sizeof(float) + static_cast<double>(vol_b) +
+                           static_cast<double>(p->workspace_bytes());
+        if (req >= static_cast<double>(1ull << 32)) {  // no sm_100a device has less than 16 GB
+            size_t free_b = 0, total_b = 0;
+            cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+            if (req >= 0.75 * static_cast<double>(total_b)) {
+                execute_host_budget(p, proj_host, vol_host, free_b > vol_b ? (free_b - vol_b) / 2 : 0, nullptr);
+                return;
+            }
         }
-        DevBuf<float> dproj, dvol;
-        dproj.alloc(proj_n, "projection stack");
-        dvol.alloc(vol_n, "volume");
+        // projections, volume and filtered stack in one allocation
+        const size_t proj_r = gct_fdk_plan::round_up(proj_n * sizeof(float)), vol_r = gct_fdk_plan::round_up(vol_b);
+        DevBuf<unsigned char> bufs;
+        bufs.alloc(proj_r + vol_r + p->stack_bytes(), "projection stack, volume and filtered stack");
+        float *const dproj = reinterpret_cast<float *>(bufs.p), *const dvol = reinterpret_cast<float *>(bufs.p + proj_r);
         cudaStream_t s = nullptr;
         cuda_check(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking), "stream");
         std::unique_ptr<CUstream_st, void (*)(cudaStream_t)> sg(s, [](cudaStream_t x) { cudaStreamDestroy(x); });
-        cuda_check(cudaMemcpyAsync(dproj.p, proj_host, proj_n * sizeof(float), cudaMemcpyHostToDevice, s),
+        cuda_check(cudaMemcpyAsync(dproj, proj_host, proj_n * sizeof(float), cudaMemcpyHostToDevice, s),
                    "projection upload");
-        execute(p, dproj.p, dvol.p, nullptr, s);
-        cuda_check(cudaMemcpyAsync(vol_host, dvol.p, vol_n * sizeof(float), cudaMemcpyDeviceToHost, s),
+        execute(p, dproj, dvol, bufs.p + proj_r + vol_r, s);
+        cuda_check(cudaMemcpyAsync(vol_host, dvol, vol_n * sizeof(float), cudaMemcpyDeviceToHost, s),
                    "volume download");
         cuda_check(cudaStreamSynchronize(s), "reconstruction");
     });

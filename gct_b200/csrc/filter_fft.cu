@@ -26,6 +26,7 @@
 // Work split: one CTA per (view, segment of quad rows) (or, for one-row detectors, per pair of
 // views). A CTA walks its rows in pairs, keeps the filtered rows of the previous pair in shared
 // memory and writes each quad row whole once its two detector rows are known.
+#include <algorithm>
 #include <cstdint>
 
 #include "../../include/gct_fdk.h"
@@ -768,7 +769,46 @@ __global__ void view_scales_kernel(const float *amax, int nv, float l1, float *v
     vinv[v] = exp2f(-e);
 }
 
+// One thread per weight. FP64 steps as in parker_table, each rounded by itself, so that a weight falls
+// into the same window; sin() may differ in the last bit. 184 000 weights took the host 2 ms.
+__global__ void parker_kernel(const double *__restrict__ gamma, const double *__restrict__ rel, double phi,
+                              float constant, int nv, int nc, float *__restrict__ out)
+{
+    constexpr double kPi = 3.14159265358979323846;
+    const long long n = static_cast<long long>(nv) * nc;
+    for (long long e = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x; e < n;
+         e += static_cast<long long>(gridDim.x) * blockDim.x) {
+        if (!gamma) {
+            out[e] = constant;
+            continue;
+        }
+        const int v = static_cast<int>(e / nc), c = static_cast<int>(e - static_cast<long long>(v) * nc);
+        const double b = rel[v], g2 = 2.0 * gamma[c];
+        const double t2 = __dadd_rn(__dadd_rn(g2, phi), -kPi), t3 = __dadd_rn(g2, kPi);
+        const double p2 = 2.0 * __dadd_rn(phi, -kPi), g4 = 2.0 * g2;
+        double w = 0.0;
+        if (b >= 0.0 && b <= t2) {
+            const double s = sin(__ddiv_rn(__dmul_rn(kPi, b), __dadd_rn(p2, g4)));
+            w = __dmul_rn(s, s);
+        } else if (b >= t2 && b <= t3) {
+            w = 1.0;
+        } else if (b >= t3 && b <= phi) {
+            const double s = sin(__ddiv_rn(__dmul_rn(kPi, __dadd_rn(phi, -b)), __dadd_rn(p2, -g4)));
+            w = __dmul_rn(s, s);
+        }
+        out[e] = static_cast<float>(w);
+    }
+}
+
 }  // namespace
+
+void launch_parker(const double *gamma, const double *rel, double phi, float constant, int nv, int nc, float *out,
+                   cudaStream_t s)
+{
+    const long long n = static_cast<long long>(nv) * nc;
+    const long long grid = std::min<long long>((n + 255) / 256, 148LL * 16);
+    parker_kernel<<<static_cast<unsigned>(grid < 1 ? 1 : grid), 256, 0, s>>>(gamma, rel, phi, constant, nv, nc, out);
+}
 
 void launch_filter_fft(const FilterArgs &a, int L, int num_sms, cudaStream_t s)
 {

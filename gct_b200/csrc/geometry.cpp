@@ -257,31 +257,41 @@ std::vector<double> ramp_taps(gct_geom_kind kind, const gct_detector &det_row,
 // src/cuda/recon/parker_weighting.cuh:19-58 (fanAngle, fanAngleDet), :80-105 (parkerWeightFan),
 // :132-176 (getParkerWeights; fan angles from view 0, relative angles reversed for CCW, weights
 // only when the range exceeds pi) and :181-200 (parallel kinds: 1 or 0.5).
-std::vector<double> parker_table(const gct_ct_geom &g, const RotationInfo &ri)
+ParkerRule parker_rule(const gct_ct_geom &g, const RotationInfo &ri)
 {
     const auto kind = static_cast<gct_geom_kind>(g.kind);
-    const unsigned nc = g.det_row.num_samples, nv = g.num_views;
-    std::vector<double> w(static_cast<size_t>(nc) * nv, 1.0);
+    const unsigned nc = g.det_row.num_samples;
+    ParkerRule r;
     if (family_of(kind) == Family::Affine) {
         const bool half = ri.incr > 0.0 && ri.range <= ri.incr + kPi;
-        std::fill(w.begin(), w.end(), half ? 1.0 : 0.5);
-        return w;
+        r.constant = half ? 1.0 : 0.5;
+        return r;
     }
-    if (!(ri.range > kPi)) return w;  // reference leaves these uninitialised; defined as 1 here
+    if (!(ri.range > kPi)) return r;  // reference leaves these uninitialised; defined as 1 here
     const gct_view_geom &v0 = g.views[0];
     const bool arc = kind == GCT_GEOM_FAN_ARC || kind == GCT_GEOM_CONE_CYL;
-    std::vector<double> gamma(nc);
+    r.gamma.resize(nc);
     for (unsigned c = 0; c < nc; ++c) {
         const double t = (static_cast<double>(c) - v0.det_row_center) * g.det_row.sampling_width;
-        gamma[c] = arc ? t : std::atan2(t, v0.src_det_dist);
+        r.gamma[c] = arc ? t : std::atan2(t, v0.src_det_dist);
     }
-    std::vector<double> rel = ri.rel_rot_ang;
-    if (ri.dir == GCT_ROT_CCW) std::reverse(rel.begin(), rel.end());
-    const double phi = ri.range;
+    r.rel = ri.rel_rot_ang;
+    if (ri.dir == GCT_ROT_CCW) std::reverse(r.rel.begin(), r.rel.end());
+    r.phi = ri.range;
+    return r;
+}
+
+std::vector<double> parker_table(const gct_ct_geom &g, const RotationInfo &ri)
+{
+    const unsigned nc = g.det_row.num_samples, nv = g.num_views;
+    const ParkerRule r = parker_rule(g, ri);
+    std::vector<double> w(static_cast<size_t>(nc) * nv, r.constant);
+    if (r.gamma.empty()) return w;
+    const double phi = r.phi;
     for (unsigned v = 0; v < nv; ++v) {
-        const double b = rel[v];
+        const double b = r.rel[v];
         for (unsigned c = 0; c < nc; ++c) {
-            const double gm = gamma[c];
+            const double gm = r.gamma[c];
             const double t2 = 2.0 * gm + phi - kPi, t3 = 2.0 * gm + kPi, t4 = phi;
             double wt = 0.0;
             if (b >= 0.0 && b <= t2) {
@@ -315,22 +325,24 @@ std::vector<std::complex<double>> filter_spectrum(const std::vector<double> &tap
         const int off = j - n / 2;
         hc[static_cast<unsigned>((off % static_cast<int>(L) + static_cast<int>(L)) % static_cast<int>(L))] += taps[j];
     }
-    std::vector<double> cs(L), sn(L);
-    for (unsigned m = 0; m < L; ++m) {
-        cs[m] = std::cos(kTwoPi * m / L);
-        sn[m] = std::sin(kTwoPi * m / L);
-    }
-    std::vector<std::complex<double>> H(L);
-    for (unsigned k = 0; k < L; ++k) {
-        double re = 0.0, im = 0.0;
-        for (unsigned m = 0; m < L; ++m) {
-            if (hc[m] == 0.0) continue;
-            const unsigned idx = static_cast<unsigned>((static_cast<unsigned long long>(k) * m) % L);
-            re += hc[m] * cs[idx];
-            im -= hc[m] * sn[idx];
+    // radix-2 transform in place, input in bit-reversed order
+    std::vector<std::complex<double>> H(L), w(L / 2);
+    for (unsigned m = 0; m < L / 2; ++m) w[m] = {std::cos(kTwoPi * m / L), -std::sin(kTwoPi * m / L)};
+    for (unsigned m = 0, r = 0; m < L; ++m) {
+        H[r] = hc[m];
+        for (unsigned bit = L >> 1; bit && ((r ^= bit) & bit) == 0; bit >>= 1) {
         }
-        H[k] = std::complex<double>(re / L, im / L);
     }
+    for (unsigned half = 1; half < L; half *= 2)
+        for (unsigned b = 0; b < L; b += 2 * half)
+            for (unsigned k = 0; k < half; ++k) {
+                const std::complex<double> u = H[b + k], t = w[k * (L / (2 * half))], x = H[b + k + half];
+                const std::complex<double> p(x.real() * t.real() - x.imag() * t.imag(),
+                                             x.real() * t.imag() + x.imag() * t.real());
+                H[b + k] = u + p;
+                H[b + k + half] = u - p;
+            }
+    for (auto &h : H) h /= static_cast<double>(L);
     return H;
 }
 

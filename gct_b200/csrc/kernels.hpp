@@ -65,6 +65,11 @@ void launch_view_absmax(const float *proj, int nv, long long pix_per_view, float
 void launch_view_scales(const float *amax, int nv, float l1, float *vscale, float *vinv,
                         cudaStream_t s);
 
+// The weights parker_table gives for Parker's windows (gamma [nc], rel [nv] on the device), or the
+// constant where gamma is NULL.
+void launch_parker(const double *gamma, const double *rel, double phi, float constant, int nv, int nc, float *out,
+                   cudaStream_t s);
+
 struct BpArgs {
     const void *quads = nullptr;
     int qpitch = 0;                // nc + 4

@@ -108,11 +108,13 @@ struct gct_fdk_plan {
     // spiral scans: per-slice view windows (first, count); count 0 leaves the slice zero
     bool spiral = false;
     DevBuf<int2> slice_views;
-    DevBuf<float4> fview;
-    DevBuf<float> parker;
-    DevBuf<float2> H;
+    // tables uploaded once, in one buffer
+    DevBuf<unsigned char> tables;
+    float4 *fview = nullptr;
+    float *parker = nullptr;
+    float2 *H = nullptr;
     DevBuf<float> bp_part;  // partial images of view-split backprojections (run_backproject)
-    DevBuf<float> coefs;
+    float *coefs = nullptr;
     DevBuf<unsigned char> work;
     // Toeplitz-GEMM filter: B = T^T split into 16-bit hi/lo pieces [Np][Kp] (BF16, or FP16 bit
     // patterns in the FP16 form), A rows [nv*nr][Kp], FP32 rows
@@ -122,7 +124,7 @@ struct gct_fdk_plan {
     DevBuf<float> grinv;             // FP16 form: per-row inverse scale of the GEMM rows
     float tap_inv = 1.f;             // FP16 form: inverse of the taps' power-of-two scale
     DevBuf<float> ybuf;
-    DevBuf<int> gemm_err;  // kernel status word (GEMM pipeline and FFT input waits)
+    int *gemm_err = nullptr;  // kernel status word (GEMM pipeline and FFT input waits)
     // staging for gct_fdk_execute_host: projections, two device volumes (consecutive calls
     // alternate, so one call's download overlaps the next call's backprojection)
     DevBuf<float> host_proj, host_vol, host_vol2;
