@@ -248,7 +248,14 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
     const bool f16 = p->opts.storage == GCT_STORAGE_F16;
     // row-pair plans have a fixed shape of their own (rows.cu); their options are checked all the same
     const bool par1d = kind == GCT_GEOM_PARALLEL_1D;
-    p->zpt = p->opts.z_per_thread > 0 ? p->opts.z_per_thread : (vol3d ? 16 : 1);
+    // FP32 quads, 4 x 16 blocks: 8 voxels per thread for the parallel kinds (256 x 256 x 160 / 300 views: 3.46
+    // against 3.80 ms) and for flat panels over at most 256 x 256 columns (256^3 / 360 views 4.30 against
+    // 4.40, short scan 253 x 241 x 187 2.82 against 2.95); larger grids lose (381 x 381 x 290 / 500 views 16.9
+    // against 16.0, 512^3 72.1 against 70.2), and so do arcs (381 x 379 x 61 / 577 views 5.6 against 5.4)
+    const bool shallow = !f16 && (p->family == gct::Family::Affine ||
+                                  (p->family == gct::Family::Projective && p->z_affine &&
+                                   static_cast<long long>(p->kx) * p->ky <= 256 * 256));
+    p->zpt = p->opts.z_per_thread > 0 ? p->opts.z_per_thread : vol3d ? (shallow ? 8 : 16) : 1;
     if (p->zpt != 1 && p->zpt != 2 && p->zpt != 4 && p->zpt != 8 && p->zpt != 16)
         gct::fail(GCT_ERR_INVALID_ARG, "z_per_thread must be 1, 2, 4, 8 or 16");
     p->bx = p->opts.block_x > 0 ? p->opts.block_x : (par1d ? 128 : vol3d ? (f16 ? 8 : 4) : 32);

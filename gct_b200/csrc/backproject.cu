@@ -46,6 +46,22 @@ constexpr int kShiftBits = 0x4B400000;  // bit pattern of kShift
 // Each affine form is c0 + ci*i + cj*j + ck*k in voxel indices.
 __device__ __forceinline__ int wscale_slot(int family) { return family == 0 ? 5 : family == 1 ? 12 : 16; }
 
+// Quad loads ask L2 for whole 256 bytes: a block's next rows and views' neighbours lie there, and fewer
+// gathers wait for DRAM (FP32 quads 512^3 / 720 views 71.4 -> 70.2 ms, 256^3 / 360 views 4.48 -> 4.40; FP16 short
+// scan 34.8 -> 34.6).
+__device__ __forceinline__ uint2 ldg_quad(const uint2 *p)
+{
+    uint2 r;
+    asm("ld.global.nc.L2::256B.v2.u32 {%0, %1}, [%2];" : "=r"(r.x), "=r"(r.y) : "l"(p));
+    return r;
+}
+__device__ __forceinline__ float4 ldg_quad(const float4 *p)
+{
+    float4 r;
+    asm("ld.global.nc.L2::256B.v4.f32 {%0, %1, %2, %3}, [%4];" : "=f"(r.x), "=f"(r.y), "=f"(r.z), "=f"(r.w) : "l"(p));
+    return r;
+}
+
 // Bilinear value of a stored coefficient quad (A, B, C, D) at column fraction fu in [0, 1] and
 // centred row fraction fvc in [-0.5, 0.5]: (A + fu B) + fvc (C + fu D). The per-column form of fu
 // (U) is precomputed once per view.
@@ -139,7 +155,7 @@ __device__ __forceinline__ void column(unsigned long long base, int stride, type
                 base + static_cast<unsigned long long>(static_cast<long long>(__float_as_int(t.x)) * stride));
             const auto *p1 = reinterpret_cast<const typename L::S *>(
                 base + static_cast<unsigned long long>(static_cast<long long>(__float_as_int(t.y)) * stride));
-            const float2 val = make_float2(L::lerp(__ldg(p0), fu, fvc.x), L::lerp(__ldg(p1), fu, fvc.y));
+            const float2 val = make_float2(L::lerp(ldg_quad(p0), fu, fvc.x), L::lerp(ldg_quad(p1), fu, fvc.y));
             const float2 r = __ffma2_rn(wt.at2(z), val, make_float2(acc[z], acc[z + 1]));
             if (!SOME || ((on >> z) & 1u)) acc[z] = r.x;
             if (!SOME || ((on >> z) & 2u)) acc[z + 1] = r.y;
@@ -153,13 +169,13 @@ __device__ __forceinline__ void column(unsigned long long base, int stride, type
                         base + static_cast<unsigned long long>(static_cast<long long>(__float_as_int(tm.x)) * stride));
                     const auto *q1 = reinterpret_cast<const typename L::S *>(
                         base + static_cast<unsigned long long>(static_cast<long long>(__float_as_int(tm.y)) * stride));
-                    valm = make_float2(L::lerp(__ldg(q0), fu, fvm.x), L::lerp(__ldg(q1), fu, fvm.y));
+                    valm = make_float2(L::lerp(ldg_quad(q0), fu, fvm.x), L::lerp(ldg_quad(q1), fu, fvm.y));
                 } else {
                     const auto *q0 = reinterpret_cast<const typename L::S *>(
                         mbase - static_cast<unsigned long long>(static_cast<long long>(__float_as_int(t.x)) * stride));
                     const auto *q1 = reinterpret_cast<const typename L::S *>(
                         mbase - static_cast<unsigned long long>(static_cast<long long>(__float_as_int(t.y)) * stride));
-                    valm = make_float2(L::lerp(__ldg(q0), fu, -fvc.x), L::lerp(__ldg(q1), fu, -fvc.y));
+                    valm = make_float2(L::lerp(ldg_quad(q0), fu, -fvc.x), L::lerp(ldg_quad(q1), fu, -fvc.y));
                 }
                 float(&dm)[ZPT] = *accm;
                 const float2 rm = __ffma2_rn(wt.at2(z), valm, make_float2(dm[z], dm[z + 1]));
@@ -176,7 +192,7 @@ __device__ __forceinline__ void column(unsigned long long base, int stride, type
             const float fvc = vm - (t - kShift);
             const auto *p = reinterpret_cast<const typename L::S *>(
                 base + static_cast<unsigned long long>(static_cast<long long>(__float_as_int(t)) * stride));
-            acc[z] = fmaf(wt.at(z), L::lerp(__ldg(p), fu, fvc), acc[z]);
+            acc[z] = fmaf(wt.at(z), L::lerp(ldg_quad(p), fu, fvc), acc[z]);
         }
     }
 }
@@ -637,7 +653,7 @@ struct ArcWeight4 {
 // bytes (FP16) or 64 bytes (FP32), 32-byte aligned, read through the non-coherent path.
 __device__ __forceinline__ void ldg_partners(unsigned long long p, uint2 (&o)[4])
 {
-    asm("ld.global.nc.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+    asm("ld.global.nc.L2::256B.v8.u32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
         : "=r"(o[0].x), "=r"(o[0].y), "=r"(o[1].x), "=r"(o[1].y), "=r"(o[2].x), "=r"(o[2].y), "=r"(o[3].x),
           "=r"(o[3].y)
         : "l"(p));
