@@ -152,9 +152,11 @@ constexpr double kEdge = 1.0 / 1024.0;
 constexpr float kFloorShift = 12582912.0f;  // 1.5 * 2^23
 constexpr int kFloorBits = 0x4B400000;
 
-__device__ __forceinline__ float2 lerp2(float2 a, float2 b, float2 f)
+// (1 - f) a + f b with g = 1 - f. Infinite taps of either sign stay what the sum of the weighted taps
+// makes of them (a + f (b - a) would turn them into NaN).
+__device__ __forceinline__ float2 lerp2(float2 a, float2 b, float2 f, float2 g)
 {
-    return __ffma2_rn(f, __ffma2_rn(a, make_float2(-1.f, -1.f), b), a);
+    return __ffma2_rn(f, b, __fmul2_rn(g, a));
 }
 
 // Sum of one ray; every lane of the warp calls it (`on` false: the lane has no ray). `grid` holds the
@@ -258,13 +260,14 @@ __device__ __forceinline__ float forward_ray(const Ray &ray, bool on, const floa
                                                   static_cast<long long>(kFloorBits) * (1LL + sy + (PLANAR ? 0 : sz))));
         // samples k and k + 1 as packed pairs at (FP32) chunk positions fk
         auto pair = [&](float2 fk) -> float2 {
-            float2 f[NA];
+            float2 f[NA], g[NA];
             Off o0 = base, o1 = base;
 #pragma unroll
             for (int a = 0; a < NA; ++a) {
                 const float2 x = __ffma2_rn(fk, make_float2(d[a], d[a]), make_float2(r[a], r[a]));
                 const float2 t = __fadd2_rd(x, make_float2(kFloorShift, kFloorShift));  // floor(x) in the low bits
                 f[a] = __ffma2_rn(__fadd2_rn(t, make_float2(-kFloorShift, -kFloorShift)), make_float2(-1.f, -1.f), x);
+                g[a] = __ffma2_rn(f[a], make_float2(-1.f, -1.f), make_float2(1.f, 1.f));
                 const Off st = a == 0 ? kVox : static_cast<Off>(static_cast<long long>(kVox) * (a == 1 ? sy : sz));
                 o0 += static_cast<Off>(__float_as_int(t.x)) * st;
                 o1 += static_cast<Off>(__float_as_int(t.y)) * st;
@@ -273,19 +276,21 @@ __device__ __forceinline__ float forward_ray(const Ray &ray, bool on, const floa
                 // (z, z + 1) pairs of four taps per sample
                 const float2 p00 = at2(b00, o0), p01 = at2(b00 + 8, o0), p10 = at2(b01, o0), p11 = at2(b01 + 8, o0);
                 const float2 q00 = at2(b00, o1), q01 = at2(b00 + 8, o1), q10 = at2(b01, o1), q11 = at2(b01 + 8, o1);
-                const float2 x0 = make_float2(f[0].x, f[0].x), y0 = make_float2(f[1].x, f[1].x);
-                const float2 x1 = make_float2(f[0].y, f[0].y), y1 = make_float2(f[1].y, f[1].y);
-                const float2 e0 = lerp2(lerp2(p00, p01, x0), lerp2(p10, p11, x0), y0);
-                const float2 e1 = lerp2(lerp2(q00, q01, x1), lerp2(q10, q11, x1), y1);
-                return lerp2(make_float2(e0.x, e1.x), make_float2(e0.y, e1.y), f[NA - 1]);
+                const auto two = [](float v) { return make_float2(v, v); };
+                const float2 x0 = two(f[0].x), y0 = two(f[1].x), x1 = two(f[0].y), y1 = two(f[1].y);
+                const float2 gx0 = two(g[0].x), gy0 = two(g[1].x), gx1 = two(g[0].y), gy1 = two(g[1].y);
+                const float2 e0 = lerp2(lerp2(p00, p01, x0, gx0), lerp2(p10, p11, x0, gx0), y0, gy0);
+                const float2 e1 = lerp2(lerp2(q00, q01, x1, gx1), lerp2(q10, q11, x1, gx1), y1, gy1);
+                return lerp2(make_float2(e0.x, e1.x), make_float2(e0.y, e1.y), f[NA - 1], g[NA - 1]);
             } else {
                 const float2 v00 = make_float2(at(b00, o0), at(b00, o1)), v01 = make_float2(at(b00 + 4, o0), at(b00 + 4, o1));
                 const float2 v10 = make_float2(at(b01, o0), at(b01, o1)), v11 = make_float2(at(b01 + 4, o0), at(b01 + 4, o1));
-                const float2 e = lerp2(lerp2(v00, v01, f[0]), lerp2(v10, v11, f[0]), f[1]);
+                const float2 e = lerp2(lerp2(v00, v01, f[0], g[0]), lerp2(v10, v11, f[0], g[0]), f[1], g[1]);
                 if constexpr (PLANAR) return e;
                 const float2 w00 = make_float2(at(b10, o0), at(b10, o1)), w01 = make_float2(at(b10 + 4, o0), at(b10 + 4, o1));
                 const float2 w10 = make_float2(at(b11, o0), at(b11, o1)), w11 = make_float2(at(b11 + 4, o0), at(b11 + 4, o1));
-                return lerp2(e, lerp2(lerp2(w00, w01, f[0]), lerp2(w10, w11, f[0]), f[1]), f[NA - 1]);
+                return lerp2(e, lerp2(lerp2(w00, w01, f[0], g[0]), lerp2(w10, w11, f[0], g[0]), f[1], g[1]), f[NA - 1],
+                             g[NA - 1]);
             }
         };
         const float lo = static_cast<float>(max(ka - k0, 0)), hi = static_cast<float>(min(kb - k0, kChunk) - 1);
