@@ -464,7 +464,10 @@ gct::BpArgs bp_args(const gct_fdk_plan *p, const StackRef &st, float *vol, int v
     ba.v_begin = v_begin;
     ba.v_count = v_count;
     ba.quarter = p->rows && p->sym ? p->nv / 4 : st.quarter;
-    if (p->rows) ba.sym = p->sym;
+    if (p->rows) {
+        ba.sym = p->sym;
+        ba.partners = st.quarter > 0 ? 1 : 0;
+    }
     ba.slice_views = p->slice_views.p;
     ba.vol = vol;
     ba.nx = p->kx;
@@ -548,6 +551,11 @@ void run_backproject_sym(gct_fdk_plan *p, const StackRef &st, float *vol, int b_
     gct::BpArgs ba = bp_args(p, st, vol, b_begin, b_count);
     ba.accumulate = accumulate ? 1 : 0;
     ba.sym = p->sym;
+    if (p->rows) {
+        gct::launch_backproject_rows_sym(ba, p->num_sms, s);
+        cuda_check(cudaGetLastError(), "backprojection kernel launch");
+        return;
+    }
     const int h = p->kx / 2;
     const long long blocks =
         static_cast<long long>((h + p->bx_sym - 1) / p->bx_sym) * ((h + p->by_sym - 1) / p->by_sym);
@@ -609,6 +617,10 @@ void prepare_partners(gct_fdk_plan *p, const float *proj, const StackRef &st, in
     if (n <= 0 || m <= 0) return;
     const bool f16 = p->opts.storage == GCT_STORAGE_F16;
     const bool whole = b == 0 && n == m;
+    if (p->rows) {  // the filter writes the interleaved rows itself
+        for (int q = 0; q < (whole ? 1 : 4); ++q) prepare(p, proj, st, whole ? 0 : b + q * m, whole ? p->nv : n, s);
+        return;
+    }
     const bool fuse = f16 && p->opts.filter != GCT_FILTER_FFT;  // the split pass finds the maxima
     if (fuse && gct::gemm_quad_tiles(static_cast<long long>(n) * p->nr, 4) >= p->num_sms) {
         // FP16 quads from the Toeplitz GEMM: rows split in partner-interleaved order (with the view

@@ -310,7 +310,8 @@ void build_batch(gct_fdk_batch *b, const gct_batch_item *items, uint32_t n, cons
         it->vol = src.vol_dev;
         it->ws.alloc(src.plan->stack_bytes(), "batch item workspace");
         // quarter-turn plans keep their interleaved partner stacks and run in the quarter-turn queue
-        it->st = stack_of(src.plan, it->ws.p, false);
+        // (row pairs stay view-major: the planar queue takes one view at a time)
+        it->st = stack_of(src.plan, it->ws.p, src.plan->rows);
         b->items.push_back(std::move(it));
     }
     // filter stages: items of one plan share its filter scratch, so they run on one side stream

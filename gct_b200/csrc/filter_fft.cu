@@ -345,8 +345,11 @@ __device__ __forceinline__ void write_row_pairs(const FilterArgs &a, int v, cons
 {
     const int pitch = a.nc + 2 * kQuadPad;
     const bool centred = a.kind == GCT_GEOM_PARALLEL_1D;
+    long long first;
+    int step;
+    quad_layout(v, pitch, a.quarter, first, step);
     for (int e = t; e < pitch; e += nthr)
-        store_row_pair<MODE == kOutRowsF16>(a.out, static_cast<long long>(v) * pitch + e, y[e], y[e + 1], centred);
+        store_row_pair<MODE == kOutRowsF16>(a.out, first + static_cast<long long>(e) * step, y[e], y[e + 1], centred);
 }
 
 // Loads, weights and packs detector rows a (real part) and b (imaginary part) at columns t + T m;

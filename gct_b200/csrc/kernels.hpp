@@ -48,7 +48,8 @@ __host__ __device__ inline void quad_layout(long long v, long long qview, int qu
 
 // Row pairs: the stack of planar kinds (1D parallel, fan line, fan arc), whose views are one row. Entry c of a view, for c in [-2, nc + 2), is (y[c], y[c + 1] - y[c]), for the
 // parallel kind ((y[c] + y[c + 1]) / 2, y[c + 1] - y[c]), with zeros outside the row, as float2 or half2
-// (scaled as the quads); views follow each other nc + 4 entries apart. With FP16 storage the
+// (scaled as the quads); views follow each other nc + 4 entries apart, or (FP16 lines with
+// the quarter-turn symmetry) partner views are interleaved as in quad_layout. With FP16 storage the
 // fans keep quads in two cases: arcs, whose blends round the column fraction to half precision, which
 // turns last-bit differences of the angle into differences of a 2048th sample, so they stay with
 // atan2f and the quarter-turn kernel that shares it between four updates; and lines with a Toeplitz
@@ -82,6 +83,7 @@ struct BpArgs {
     float umax = 0.f, vmax = 0.f;  // nc, nr
     int accumulate = 0;
     int quarter = 0;  // quad_layout of the stack
+    int partners = 0;  // row pairs: interleaved partner views (FP16 lines)
     // spiral scans (one voxel per thread along z): slice k backprojects views [x, x + y) of
     // slice_views[k], intersected with [v_begin, v_begin + v_count)
     const int2 *slice_views = nullptr;
@@ -115,8 +117,12 @@ void launch_backproject_sym(const BpArgs &a, int family, int storage, int zpt, i
 
 // Planar kinds over row pairs (rows.cu): views [a.v_begin, a.v_begin + a.v_count) into the image.
 // a.quads, a.qview: the pairs and the entries per view; a.sym, a.quarter: quarter-turn plans, whose
-// view v takes its coordinates from base view v mod quarter at the turned pixel (view-major all the same).
+// view v takes its coordinates from base view v mod quarter at the turned pixel; a.partners: the pairs of
+// partner views are interleaved (quad_layout), else view-major.
 void launch_backproject_rows(const BpArgs &a, int family, int storage, int num_sms, cudaStream_t s);
+// Quarter-turn plans over interleaved partner rows (a.partners): base views [a.v_begin, + a.v_count) and
+// their partners.
+void launch_backproject_rows_sym(const BpArgs &a, int num_sms, cudaStream_t s);
 // Filtered rows Y (nc apart) of views [v0, v0 + nv) -> row pairs of the stack `out`; vscale: FP16.
 void launch_row_pairs(const float *Y, int v0, int nv, int nc, bool centred, const float *vscale, void *out,
                       int num_sms, cudaStream_t s);

@@ -158,6 +158,8 @@ struct gct_fdk_plan {
     {
         return static_cast<size_t>(nr + 2 * gct::kQuadPad) * (nc + 2 * gct::kQuadPad) * quad_bytes();
     }
+    // Row pairs of quarter-turn FP16 lines interleave the partner views
+    bool partner_rows() const { return rows && sym && family == gct::Family::Projective && opts.storage == GCT_STORAGE_F16; }
     // Bytes between the views of a stack: row pairs take a part of view_bytes(), which budgets and the
     // published workspace size keep counting with.
     size_t view_stride() const
@@ -187,7 +189,7 @@ inline StackRef stack_of(const gct_fdk_plan *p, void *workspace, bool view_major
 {
     StackRef r;
     r.quads = static_cast<unsigned char *>(workspace);
-    r.quarter = (p->sym && !p->rows && !view_major) ? p->nv / 4 : 0;
+    r.quarter = (p->sym && (!p->rows || p->partner_rows()) && !view_major) ? p->nv / 4 : 0;
     if (p->opts.storage == GCT_STORAGE_F16) {
         r.amax = reinterpret_cast<float *>(r.quads + p->quad_region());
         r.vscale = r.amax + p->nv;

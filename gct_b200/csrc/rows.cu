@@ -11,16 +11,19 @@
 // storage blends in half precision as they do: the rounding of a coordinate of 2000 samples is most of
 // an image's error, and it stays what it was.
 //
-// Bound by instruction issue: about 7 (parallel), 10 (line) and 17 (arc) instructions per update.
+// Bound by instruction issue: 11 (parallel), 16 (FP16 line) and 23 (arc) instructions per update at 58 to 64 % of
+// the issue slots (the arc's polynomial also fills the FMA pipe).
 // Filter and backprojection, against the quad kernels over one-row views: parallel 1024 x 1024, 900 views
 // of 1455: 1.81 -> 0.47 ms; arc 509 x 387, 1151 views of 671: 1.13 -> 0.28 ms; line 512 x 512, 720 views
-// of 768, FP16: 0.208 -> 0.161 ms.
+// of 768, FP16: 0.208 -> 0.161 ms (0.114 with the quarter-turn form below).
 // Cells per image are few (1024^2: 1024), so the views of a cell are cut into up to eight chunks, one
 // per block of a thread-block cluster; the blocks sum their parts through distributed shared memory
 // in chunk order and each writes its share of the cell, so there are no partial images and the
 // result does not depend on timing.
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
+
+#include <type_traits>
 
 #include "../../include/gct_fdk.h"
 #include "common.cuh"
@@ -92,6 +95,11 @@ struct RowF16 {
         }
         return __half22float2(__hfma2(__floats2half2_rn(f.x, f.y), __highs2half2(h0, h1), __lows2half2(h0, h1)));
     }
+};
+
+// One partner of an interleaved stack, for launches over some of the views only.
+struct RowF16Partner : RowF16 {
+    static constexpr unsigned kBytes = 16;
 };
 
 // Adds one view to the thread's pixels. INSIDE: the cell's samples lie well inside the row (and in
@@ -240,7 +248,9 @@ __device__ __forceinline__ void cell_sums(const BpArgs &a, int i0, int j0, int t
             __syncthreads();
             if (tid < nvc) stage_view<FAMILY>(a, v + tid, v + tid - q * (SYM ? a.quarter : 0), box, s_view[tid]);
             __syncthreads();
-            const char *row = static_cast<const char *>(a.quads) + static_cast<long long>(v) * row_bytes;
+            const char *row = static_cast<const char *>(a.quads);
+            if (R::kBytes == RowF16Partner::kBytes) row += static_cast<long long>(v - q * a.quarter) * row_bytes + 4 * q;
+            else row += static_cast<long long>(v) * row_bytes;
             for (int k = 0; k < nvc; ++k, row += row_bytes) {
                 const int cls = s_view[k].cls;
                 if (cls == kOff) continue;  // every pixel of the cell would add zero
@@ -351,6 +361,148 @@ __global__ void __launch_bounds__(kQueueThreads, 4)
     }
 }
 
+// ---- quarter-turn plans, FP16 lines -------------------------------------------------------------
+//
+// The rows of the four partner views are interleaved entry by entry (16 bytes). A thread owns the four
+// columns R^k(c) of four first-quadrant pixels c and, per base view, evaluates the coordinates at each
+// R^k(c) once for the four partners (partner q adds to column R^(k+q)(c)): one 16-byte load and one
+// evaluation per four updates. Cells are 32 x 16 pixels of the quadrant.
+// Bound by issue at 14 warps per SM (1024 blocks). 512 x 512 pixels, 720 views of 768: 142 us one view at a
+// time, 92 us this way (2.05 T updates/s); the call 0.161 -> 0.114 ms.
+constexpr int kSymCellY = 16, kSymPairs = 2;
+
+// Indices of R^K of pixels (i, j): var along the thread's pixels, c the other one (Pixels).
+template <int K>
+__device__ __forceinline__ void turn_pixels(int sym, float n1, float i, const float2 (&j)[kSymPairs], Pixels &px)
+{
+    const bool flip_j = K == 2 || K == (sym > 0 ? 1 : 3), flip_i = K == 2 || K == (sym > 0 ? 3 : 1);
+    px.c = flip_i ? n1 - i : i;
+#pragma unroll
+    for (int p = 0; p < kSymPairs; ++p) px.var[p] = flip_j ? make_float2(n1 - j[p].x, n1 - j[p].y) : j[p];
+}
+
+// Adds base view v's evaluation at R^K of the thread's pixels, for its four partners (weights w).
+template <int K, bool INSIDE>
+__device__ __forceinline__ void add_partners(const CellView &v, float4 w, const char *row, float umax,
+                                             const Pixels &px, float2 (&acc)[4][kSymPairs])
+{
+#pragma unroll
+    for (int p = 0; p < kSymPairs; ++p) {
+        const float2 d = form<(K & 1) != 0>(v.b, px, p);
+        const float2 inv = make_float2(rcp_approx(d.x), rcp_approx(d.y));
+        float2 u = __fmul2_rn(form<(K & 1) != 0>(v.a, px, p), inv);
+        const float2 i2 = __fmul2_rn(inv, inv);
+        bool on0 = true, on1 = true;
+        if (!INSIDE) {
+            on0 = u.x >= -1.0f && u.x <= umax;
+            on1 = u.y >= -1.0f && u.y <= umax;
+            u = make_float2(on0 ? u.x : -1.0f, on1 ? u.y : -1.0f);
+        }
+        const float2 t = __fadd2_rd(u, two(kShift));
+        const float2 f = __ffma2_rn(__fadd2_rn(t, two(-kShift)), two(-1.f), u);
+        constexpr unsigned kBase = (static_cast<unsigned>(kQuadPad) - kShiftBits) * 16u;  // modulo 2^32
+        const uint4 e0 = __ldg(reinterpret_cast<const uint4 *>(row + (__float_as_uint(t.x) * 16u + kBase)));
+        const uint4 e1 = __ldg(reinterpret_cast<const uint4 *>(row + (__float_as_uint(t.y) * 16u + kBase)));
+        const __half2 fh = __floats2half2_rn(f.x, f.y);
+        auto blend = [&](unsigned h0, unsigned h1, float wq, float2 &sum) {
+            const __half2 a0 = *reinterpret_cast<const __half2 *>(&h0), a1 = *reinterpret_cast<const __half2 *>(&h1);
+            const float2 val = __half22float2(__hfma2(fh, __highs2half2(a0, a1), __lows2half2(a0, a1)));
+            const float2 r = __ffma2_rn(__fmul2_rn(two(wq), i2), val, sum);
+            if (on0) sum.x = r.x;
+            if (on1) sum.y = r.y;
+        };
+        blend(e0.x, e1.x, w.x, acc[K][p]);
+        blend(e0.y, e1.y, w.y, acc[(K + 1) & 3][p]);
+        blend(e0.z, e1.z, w.z, acc[(K + 2) & 3][p]);
+        blend(e0.w, e1.w, w.w, acc[(K + 3) & 3][p]);
+    }
+}
+
+// A cluster of gridDim.z blocks per cell, each with its chunk of the base views [a.v_begin, + a.v_count).
+__global__ void __launch_bounds__(kThreads, 6) rows_sym_kernel(BpArgs a, int chunk)
+{
+    __shared__ CellView s_view[kStage];
+    __shared__ float4 s_w[kStage];        // weight scales of the four partners
+    __shared__ int4 s_cls[kStage];        // class of the cell's four turned images
+    __shared__ float s_sum[4][2 * kSymPairs][kThreads];
+    const int i0 = blockIdx.x * kCell, j0 = blockIdx.y * kSymCellY, tid = threadIdx.x, h = a.nx / 2;
+    const int z = blockIdx.z, chunks = gridDim.z;
+    const int v_begin = a.v_begin + z * chunk, v_end = min(v_begin + chunk, a.v_begin + a.v_count);
+    const float n1 = static_cast<float>(a.nx - 1);
+    const float i1 = static_cast<float>(min(i0 + kCell, h) - 1), j1 = static_cast<float>(min(j0 + kSymCellY, h) - 1);
+    const int lane = tid & 31;
+    // pixels past the quadrant repeat its last ones and are not stored
+    const float fi = fminf(static_cast<float>(i0 + (tid >> 5) * 8 + (lane & 7)), i1);
+    const float fy = static_cast<float>(j0 + (lane >> 3));
+    float2 fj[kSymPairs], acc[4][kSymPairs];
+#pragma unroll
+    for (int p = 0; p < kSymPairs; ++p) {
+        fj[p] = make_float2(fminf(fy + 8.f * p, j1), fminf(fy + 8.f * p + 4.f, j1));
+#pragma unroll
+        for (int k = 0; k < 4; ++k) acc[k][p] = make_float2(0.f, 0.f);
+    }
+    for (int vc = v_begin; vc < v_end; vc += kStage) {
+        const int nvc = min(kStage, v_end - vc);
+        __syncthreads();
+        if (tid / 4 < nvc) {
+            const int sv = tid / 4, k = tid & 3, v = vc + sv;
+            // the cell's box under k turns
+            const bool flip_j = k == 2 || k == (a.sym > 0 ? 1 : 3), flip_i = k == 2 || k == (a.sym > 0 ? 3 : 1);
+            Box box{static_cast<float>(i0), i1, static_cast<float>(j0), j1};
+            if (flip_i) box.i0 = n1 - i1, box.i1 = n1 - static_cast<float>(i0);
+            if (flip_j) box.j0 = n1 - j1, box.j1 = n1 - static_cast<float>(j0);
+            if (k & 1) box = Box{box.j0, box.j1, box.i0, box.i1};
+            CellView mine;
+            stage_view<1>(a, v + k * a.quarter, v, box, mine);
+            reinterpret_cast<int *>(&s_cls[sv])[k] = mine.cls;
+            reinterpret_cast<float *>(&s_w[sv])[k] = mine.a.w;
+            if (k == 0) s_view[sv] = mine;
+        }
+        __syncthreads();
+        const long long base_bytes = a.qview * 16;
+        const char *row = static_cast<const char *>(a.quads) + vc * base_bytes;
+        for (int k = 0; k < nvc; ++k, row += base_bytes) {
+            const CellView &v = s_view[k];
+            const float4 w = s_w[k];
+            const int4 cls = s_cls[k];
+            Pixels px;
+            auto add = [&](auto turn, int c) {
+                constexpr int K = decltype(turn)::value;
+                if (c == kOff) return;  // every pixel of the image would add zero
+                turn_pixels<K>(a.sym, n1, fi, fj, px);
+                if (c == kInside) add_partners<K, true>(v, w, row, a.umax, px, acc);
+                else add_partners<K, false>(v, w, row, a.umax, px, acc);
+            };
+            add(std::integral_constant<int, 0>(), cls.x);
+            add(std::integral_constant<int, 1>(), cls.y);
+            add(std::integral_constant<int, 2>(), cls.z);
+            add(std::integral_constant<int, 3>(), cls.w);
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < 4; ++k)
+#pragma unroll
+        for (int p = 0; p < 2 * kSymPairs; ++p) s_sum[k][p][tid] = (p & 1) ? acc[k][p / 2].y : acc[k][p / 2].x;
+    cg::cluster_group cl = cg::this_cluster();
+    cl.sync();
+    // the block's share of the pixels, over the chunks in order
+    for (int e = z; e < 8 * kSymPairs; e += chunks) {
+        const int k = e / (2 * kSymPairs), p = e % (2 * kSymPairs);
+        float s = 0.f;
+        for (int c = 0; c < chunks; ++c) s += *cl.map_shared_rank(&s_sum[k][p][tid], c);
+        int x = i0 + (tid >> 5) * 8 + (tid & 7), y = j0 + ((tid >> 3) & 3) + 4 * p;
+        if (x >= h || y >= h) continue;
+        for (int r = 0; r < k; ++r) {  // the plan's quarter turn
+            const int tx = a.sym > 0 ? a.nx - 1 - y : y, ty = a.sym > 0 ? x : a.nx - 1 - x;
+            x = tx;
+            y = ty;
+        }
+        float *dst = a.vol + static_cast<long long>(y) * a.nx + x;
+        *dst = a.accumulate ? *dst + s : s;
+    }
+    cl.sync();  // the sums stay until every block has read them
+}
+
 // Filtered rows Y (row stride nc, views v0 on) -> row pairs.
 template <bool F16>
 __global__ void row_pairs_kernel(const float *__restrict__ Y, int v0, int nv, int nc, bool centred,
@@ -369,12 +521,13 @@ __global__ void row_pairs_kernel(const float *__restrict__ Y, int v0, int nv, in
     }
 }
 
-template <class R>
-void launch_rows(const BpArgs &a, int family, int num_sms, cudaStream_t s)
+// Launches kern over clusters of view chunks per cell.
+template <class Kern>
+void launch_cells(Kern kern, const BpArgs &a, dim3 cells, int num_sms, cudaStream_t s)
 {
-    const dim3 cells((a.nx + kCell - 1) / kCell, (a.ny + kCell - 1) / kCell);
-    // chunks of at least 8 views until the grid holds six waves of eight blocks per SM: the last wave
-    // of a launch of one to two waves runs nearly empty
+    // chunks of at least 8 views until the grid holds six waves of eight blocks per SM: the last wave of
+    // a launch of one to two waves runs nearly empty, and chunk counts that just fill whole waves measured
+    // slower than finer ones (512 x 512 pixels one view at a time: 4 chunks 173 us, 8 chunks 142 us)
     const long long want = 6LL * 8 * num_sms;
     int chunks = 1;
     while (chunks < 8 && static_cast<long long>(cells.x) * cells.y * chunks < want && a.v_count / (2 * chunks) >= 8)
@@ -391,14 +544,21 @@ void launch_rows(const BpArgs &a, int family, int num_sms, cudaStream_t s)
     at[0].val.clusterDim.z = static_cast<unsigned>(chunks);
     cfg.attrs = at;
     cfg.numAttrs = 1;
+    cudaLaunchKernelEx(&cfg, kern, a, chunk);
+}
+
+template <class R>
+void launch_rows(const BpArgs &a, int family, int num_sms, cudaStream_t s)
+{
+    const dim3 cells((a.nx + kCell - 1) / kCell, (a.ny + kCell - 1) / kCell);
     if (family == 0) {
-        cudaLaunchKernelEx(&cfg, rows_kernel<0, R, false>, a, chunk);
+        launch_cells(rows_kernel<0, R, false>, a, cells, num_sms, s);
     } else if (family == 1) {
-        if (a.sym) cudaLaunchKernelEx(&cfg, rows_kernel<1, R, true>, a, chunk);
-        else cudaLaunchKernelEx(&cfg, rows_kernel<1, R, false>, a, chunk);
+        if (a.sym) launch_cells(rows_kernel<1, R, true>, a, cells, num_sms, s);
+        else launch_cells(rows_kernel<1, R, false>, a, cells, num_sms, s);
     } else if constexpr (R::kBytes == RowF32::kBytes) {
-        if (a.sym) cudaLaunchKernelEx(&cfg, rows_kernel<2, R, true>, a, chunk);
-        else cudaLaunchKernelEx(&cfg, rows_kernel<2, R, false>, a, chunk);
+        if (a.sym) launch_cells(rows_kernel<2, R, true>, a, cells, num_sms, s);
+        else launch_cells(rows_kernel<2, R, false>, a, cells, num_sms, s);
     }
 }
 
@@ -406,8 +566,16 @@ void launch_rows(const BpArgs &a, int family, int num_sms, cudaStream_t s)
 
 void launch_backproject_rows(const BpArgs &a, int family, int storage, int num_sms, cudaStream_t s)
 {
-    if (storage == 0) launch_rows<RowF32>(a, family, num_sms, s);
+    const dim3 cells((a.nx + kCell - 1) / kCell, (a.ny + kCell - 1) / kCell);
+    if (a.partners) launch_cells(rows_kernel<1, RowF16Partner, true>, a, cells, num_sms, s);
+    else if (storage == 0) launch_rows<RowF32>(a, family, num_sms, s);
     else launch_rows<RowF16>(a, family, num_sms, s);
+}
+
+void launch_backproject_rows_sym(const BpArgs &a, int num_sms, cudaStream_t s)
+{
+    const int h = a.nx / 2;
+    launch_cells(rows_sym_kernel, a, dim3((h + kCell - 1) / kCell, (h + kSymCellY - 1) / kSymCellY), num_sms, s);
 }
 
 int rows_queue_blocks_per_sm(int storage)

@@ -31,6 +31,10 @@ CASES = [
     ("fan_line", 129, 131, 33, 97, 1.0, (-4.0, 6.0), -1, "f32", "fft"),
     ("fan_line", 120, 60, 128, 96, 6.0, (0.0, 0.0), 1, "f32", "fft"),
     ("fan_line", 64, 96, 64, 64, 1.0, (0.0, 0.0), 1, "f16", "fft"),
+    ("fan_line", 36, 40, 2, 2, 1.0, (0.0, 0.0), 1, "f16", "fft"),  # quarter turns: partners interleaved
+    ("fan_line", 132, 90, 70, 70, 1.0, (0.0, 0.0), -1, "f16", "fft"),
+    ("fan_line", 64, 60, 96, 96, 6.0, (0.0, 0.0), 1, "f16", "fft"),
+    ("fan_line", 66, 60, 64, 64, 1.0, (0.0, 0.0), 1, "f16", "fft"),  # no quarter turns
     ("fan_arc", 9, 67, 33, 31, 1.0, (0.0, 0.0), 1, "f32", "fft"),
     ("fan_arc", 131, 128, 65, 40, 1.0, (5.0, 3.0), -1, "f32", "fft"),
     ("fan_arc", 120, 61, 96, 96, 6.0, (0.0, 0.0), 1, "f32", "fft"),
