@@ -237,7 +237,8 @@ __device__ __forceinline__ void column_dispatch(const typename L::S *view, int e
 // projective (z-affine) family. u and v are linear or linear-fractional in each index with a
 // positive denominator over the box, so their extremes are at the corners; the tests keep a
 // margin of 1/64 pixel so that the per-column values, computed with the same formulas, agree.
-template <int FAMILY>
+// COLS: the affine rows as expressions of the column, as the plain column kernel has them (bp_column).
+template <int FAMILY, bool COLS>
 __device__ __forceinline__ int box_class(const float *c, float i0, float i1, float j0, float j1, float k0, float k1,
                                          float umax, float vmax)
 {
@@ -248,8 +249,9 @@ __device__ __forceinline__ int box_class(const float *c, float i0, float i1, flo
         float u, va, vb;
         if (FAMILY == 0) {
             u = fmaf(c[2], fj, fmaf(c[1], fi, c[0]));
-            va = fmaf(c[4], k0, c[3]);
-            vb = fmaf(c[4], k1, c[3]);
+            const float V = COLS ? fmaf(c[7], fj, fmaf(c[6], fi, c[3])) : c[3];
+            va = fmaf(c[4], k0, V);
+            vb = fmaf(c[4], k1, V);
         } else {
             const float D = fmaf(c[10], fj, fmaf(c[9], fi, c[8]));
             if (!(D > 0.0f)) return kBoxMixed;
@@ -339,7 +341,7 @@ __device__ __forceinline__ void bp_column(const BpArgs &a, int i, int j, int k0,
                 float *ct = reinterpret_cast<float *>(s_coef) + t * kC;
                 if (a.vinv) ct[wscale_slot(FAMILY)] *= __ldg(a.vinv + a.v_begin + vc + t);
                 if (kClassify)
-                    s_cls[t] = box_class<FAMILY>(ct, s_box->i0, s_box->i1, s_box->j0, s_box->j1, s_box->k0, s_box->k1,
+                    s_cls[t] = box_class<FAMILY, !MIRROR>(ct, s_box->i0, s_box->i1, s_box->j0, s_box->j1, s_box->k0, s_box->k1,
                                                  a.umax, a.vmax);
             }
             __syncthreads();
@@ -355,7 +357,12 @@ __device__ __forceinline__ void bp_column(const BpArgs &a, int i, int j, int k0,
             if (FAMILY == 0) {
                 // parallel kinds: u = u0 + ui i + uj j, v = v0 + vk k, constant weight
                 const float u = fmaf(c[2], fj, fmaf(c[1], fi, c[0]));
-                const float v0 = fmaf(c[4], fk0, c[3]);
+                // The row coordinate does not depend on the column (c[6], c[7] are zero). Where a thread holds
+                // the mirror voxels too, the compiler takes the rows' splits once per block, which pays (512 x 512
+                // x 64 voxels, 575 views: 8.1 -> 6.3 ms); in the plain kernel that measured slower (FP16 7.0 against
+                // 10.3 ms, FP32 7.1 against 8.0), so there it stays an expression of the column.
+                const float v0 = MIRROR ? fmaf(c[4], fk0, c[3])
+                                        : fmaf(c[4], fk0, fmaf(c[7], fj, fmaf(c[6], fi, c[3])));
                 column_dispatch<L, ZPT, MIRROR>(view, es, a.qpitch, u, v0, c[4], a.umax, a.vmax, ConstWeight{c[5]},
                                                 acc, cls, MIRROR ? &accm : nullptr);
             } else if (FAMILY == 1) {
@@ -848,7 +855,7 @@ __device__ __forceinline__ void sym_tile(const BpArgs &a, int i0, int j0, int k0
             float4 b = box0;
 #pragma unroll
             for (int k = 0; k < 4; ++k) {
-                const int cls = kClassify ? box_class<FAMILY>(reinterpret_cast<const float *>(s_coef) + t * kC, b.x,
+                const int cls = kClassify ? box_class<FAMILY, false>(reinterpret_cast<const float *>(s_coef) + t * kC, b.x,
                                                               b.y, b.z, b.w, bk0, bk1, a.umax, a.vmax)
                                           : kBoxMixed;
                 packed |= cls << (2 * k);
