@@ -248,8 +248,8 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
     const bool f16 = p->opts.storage == GCT_STORAGE_F16;
     // row-pair plans have a fixed shape of their own (rows.cu); their options are checked all the same
     const bool par1d = kind == GCT_GEOM_PARALLEL_1D;
-    // FP32 quads, 4 x 16 blocks: 8 voxels per thread for the parallel kinds (256 x 256 x 160 / 300 views: 3.46
-    // against 3.80 ms) and for flat panels over at most 256 x 256 columns (256^3 / 360 views 4.30 against
+    // FP32 quads, 4 x 16 blocks: 8 voxels per thread for the parallel kinds (256 x 256 x 160 / 300 views: 2.84
+    // against 3.79 ms) and for flat panels over at most 256 x 256 columns (256^3 / 360 views 4.30 against
     // 4.40, short scan 253 x 241 x 187 2.82 against 2.95); larger grids lose (381 x 381 x 290 / 500 views 16.9
     // against 16.0, 512^3 72.1 against 70.2), and so do arcs (381 x 379 x 61 / 577 views 5.6 against 5.4)
     const bool shallow = !f16 && (p->family == gct::Family::Affine ||
@@ -417,8 +417,9 @@ void run_filter_gemm(gct_fdk_plan *p, const float *proj, void *out, const float 
 }  // namespace
 
 // `out` is the view-0 address of the output; `vscale` (FP16 stacks only) the view-0 scales;
-// `quarter` the quad_layout of a quad output. `fused_scales` (Toeplitz form only, amax zeroed by
-// the caller): the split pass also finds the view maxima and the scales follow it.
+// `quarter` the quad_layout of a quad output. `fused_scales`: Toeplitz form (amax zeroed by the
+// caller), the split pass also finds the view maxima and the scales follow it; FP16 row pairs with the FFT
+// (always), the filter finds the scales.
 void run_filter(gct_fdk_plan *p, const float *proj, void *out, const float *vscale, int mode, int quarter, int vb,
                 int vc, cudaStream_t s, const StackRef *fused_scales)
 {
@@ -448,7 +449,12 @@ void run_filter(gct_fdk_plan *p, const float *proj, void *out, const float *vsca
         fa.v0 = vb;
         fa.quarter = quarter;
     }
-    fa.vscale = (mode == gct::kOutQuadF16 || mode == gct::kOutRowsF16) ? vscale + vb : nullptr;
+    fa.vscale = (mode == gct::kOutQuadF16) ? vscale + vb : nullptr;
+    if (mode == gct::kOutRowsF16) {
+        fa.scale = fused_scales->vscale + vb;
+        fa.inv = fused_scales->vinv + vb;
+        fa.l1 = p->l1;
+    }
     gct::launch_filter_fft(fa, static_cast<int>(p->L), p->num_sms, s);
     cuda_check(cudaGetLastError(), "filter kernel launch");
 }
@@ -602,9 +608,10 @@ void prepare(gct_fdk_plan *p, const float *proj, const StackRef &st, int vb, int
     if (!proj) gct::fail(GCT_ERR_INVALID_ARG, "NULL projection pointer");
     if (vc <= 0) return;
     const bool f16 = p->opts.storage == GCT_STORAGE_F16;
-    const bool fuse = f16 && p->opts.filter != GCT_FILTER_FFT;  // the split pass finds the maxima
-    if (fuse) cuda_check(cudaMemsetAsync(st.amax + vb, 0, sizeof(float) * vc, s), "view maxima reset");
-    else if (f16) view_scales(p, proj, st, vb, vc, s);
+    // the split pass finds the maxima, the FFT filter of row pairs the scales
+    const bool split = f16 && p->opts.filter != GCT_FILTER_FFT, fuse = split || (f16 && p->rows);
+    if (split) cuda_check(cudaMemsetAsync(st.amax + vb, 0, sizeof(float) * vc, s), "view maxima reset");
+    else if (f16 && !fuse) view_scales(p, proj, st, vb, vc, s);
     const int mode = p->rows ? (f16 ? gct::kOutRowsF16 : gct::kOutRowsF32) : f16 ? gct::kOutQuadF16 : gct::kOutQuadF32;
     run_filter(p, proj, st.quads, st.vscale, mode, st.quarter, vb, vc, s,
                fuse ? &st : nullptr);

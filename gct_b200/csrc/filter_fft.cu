@@ -352,6 +352,15 @@ __device__ __forceinline__ void write_row_pairs(const FilterArgs &a, int v, cons
         store_row_pair<MODE == kOutRowsF16>(a.out, first + static_cast<long long>(e) * step, y[e], y[e + 1], centred);
 }
 
+// Power-of-two exponent of a view's FP16 scale. Quad coefficients are sums and differences of up to four
+// filtered values: 4 * bound is kept below 2^14 so FP16 never overflows.
+__device__ __forceinline__ float view_exponent(float amax, float l1)
+{
+    const float bound = 4.0f * amax * l1;
+    if (bound > 0.f && isfinite(bound)) return fminf(fmaxf(floorf(log2f(16384.f / bound)), -100.f), 100.f);
+    return 0.f;
+}
+
 // Loads, weights and packs detector rows a (real part) and b (imaginary part) at columns t + T m;
 // NULL rows are zero. Columns at or past nc are zero. The rows are in shared memory, the Parker rows
 // ka, kb in global memory.
@@ -545,6 +554,10 @@ __global__ void __launch_bounds__(Fft<LOG2L>::T, fft_min_blocks<LOG2L>())
     Bases<LOG2L> bs;
     bs.init(t);
     for (int e = t; e < 3 * rpitch; e += T) rows[e] = 0.f;
+    // FP16 row pairs: the raw maxima of the pair's views (a row is a whole view), as integer bits
+    constexpr bool kScales = MODE == kOutRowsF16;
+    __shared__ int s_amax[2];
+    if (kScales && t < 2) s_amax[t] = 0;
     if (BULK && t == 0) {
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bars)) : "memory");
         asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(smem_addr(bars + 1)) : "memory");
@@ -552,7 +565,6 @@ __global__ void __launch_bounds__(Fft<LOG2L>::T, fft_min_blocks<LOG2L>())
     }
     __syncthreads();
     float2 x[16];
-
     const long long items = ONE_ROW ? (a.nv + 1) / 2 : static_cast<long long>(a.nv) * nseg;
     const PairSeq q{a.nv, a.nr, seg, nseg, items, quads, ONE_ROW};
     const long long pix = static_cast<long long>(a.nr) * a.nc;
@@ -640,6 +652,19 @@ __global__ void __launch_bounds__(Fft<LOG2L>::T, fft_min_blocks<LOG2L>())
             if (pr.va >= 0) pa = st;
             if (pr.vb >= 0) pb = st + a.nc;
             ++n_used;
+            if constexpr (kScales) {  // the columns this thread copied, or any of a TMA copy
+                float ma = 0.f, mb = 0.f;
+                for (int c = t; c < a.nc; c += T) {
+                    ma = fmaxf(ma, fabsf(pa[c]));
+                    if (pb) mb = fmaxf(mb, fabsf(pb[c]));
+                }
+                constexpr unsigned kMask = T >= 32 ? 0xffffffffu : (1u << (T & 31)) - 1u;
+                const int ia = __reduce_max_sync(kMask, __float_as_int(ma)), ib = __reduce_max_sync(kMask, __float_as_int(mb));
+                if ((t & 31) == 0) {
+                    atomicMax(&s_amax[0], ia);
+                    atomicMax(&s_amax[1], ib);
+                }
+            }
             filter_pair<LOG2L, HALF>(a, x, buf, t, bs, pa, pb, pr.va, pr.ra, pr.vb, pr.rb);  // holds barriers
         }
         if constexpr (!quads) {
@@ -657,7 +682,24 @@ __global__ void __launch_bounds__(Fft<LOG2L>::T, fft_min_blocks<LOG2L>())
         } else if constexpr (ONE_ROW) {
             // each view's grid is written whole from its own row
             float *ya = rows, *yb = rows + rpitch;
-            const float s_a = a.vscale ? a.vscale[pr.va] : 1.f, s_b = (a.vscale && pr.vb >= 0) ? a.vscale[pr.vb] : 1.f;
+            float s_a = 1.f, s_b = 1.f;
+            if constexpr (kScales) {
+                const float ea = view_exponent(__int_as_float(s_amax[0]), a.l1);
+                const float eb = view_exponent(__int_as_float(s_amax[1]), a.l1);
+                s_a = exp2f(ea);
+                s_b = exp2f(eb);
+                if (t == 0) {
+                    a.scale[pr.va] = s_a;
+                    a.inv[pr.va] = exp2f(-ea);
+                    if (pr.vb >= 0) {
+                        a.scale[pr.vb] = s_b;
+                        a.inv[pr.vb] = exp2f(-eb);
+                    }
+                }
+            } else if (a.vscale) {
+                s_a = a.vscale[pr.va];
+                if (pr.vb >= 0) s_b = a.vscale[pr.vb];
+            }
             stage_rows<LOG2L>(x, ya, yb, s_a, s_b, a.nc, t);
             __syncthreads();
             for (int h = 0; h < 2; ++h) {
@@ -674,6 +716,7 @@ __global__ void __launch_bounds__(Fft<LOG2L>::T, fft_min_blocks<LOG2L>())
                     write_quad_row<MODE>(a, a.v0 + v, 2, nullptr, nullptr, t, T);
                 }
             }
+            if (kScales && t < 2) s_amax[t] = 0;  // read by all before the barrier above
             __syncthreads();  // the shared rows are rewritten by the next pair
         } else {
             // quad rows [q0, q1) of view v: quad row r needs detector rows r and r + 1
@@ -789,11 +832,7 @@ __global__ void view_scales_kernel(const float *amax, int nv, float l1, float *v
 {
     const int v = blockIdx.x * blockDim.x + threadIdx.x;
     if (v >= nv) return;
-    // quad coefficients are sums and differences of up to four filtered values: keep 4 * bound
-    // below 2^14 so FP16 never overflows
-    const float bound = 4.0f * amax[v] * l1;
-    float e = 0.f;
-    if (bound > 0.f && isfinite(bound)) e = fminf(fmaxf(floorf(log2f(16384.f / bound)), -100.f), 100.f);
+    const float e = view_exponent(amax[v], l1);
     vscale[v] = exp2f(e);
     vinv[v] = exp2f(-e);
 }

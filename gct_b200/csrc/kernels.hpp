@@ -24,6 +24,10 @@ struct FilterArgs {
     int v0 = 0;                    // quads, row pairs: stack index of the first view filtered
     int quarter = 0;               // quads: quad_layout's quarter
     const float *vscale = nullptr; // per-view output scale for quads and row pairs (nullable = 1)
+    // FP16 row pairs: the filter finds the views' scales itself (launch_view_scales' rule with l1) and writes
+    // them and their inverses here, view 0 of the launch
+    float *scale = nullptr, *inv = nullptr;
+    float l1 = 0.f;
     int *err = nullptr;            // plan status word: kFftWaitTimeout when an input copy timed out
 };
 

@@ -15,7 +15,7 @@
 // the issue slots (the arc's polynomial also fills the FMA pipe).
 // Filter and backprojection, against the quad kernels over one-row views: parallel 1024 x 1024, 900 views
 // of 1455: 1.81 -> 0.47 ms; arc 509 x 387, 1151 views of 671: 1.13 -> 0.28 ms; line 512 x 512, 720 views
-// of 768, FP16: 0.208 -> 0.161 ms (0.114 with the quarter-turn form below).
+// of 768, FP16: 0.208 -> 0.161 ms (0.104 with the quarter-turn form below).
 // Cells per image are few (1024^2: 1024), so the views of a cell are cut into up to eight chunks, one
 // per block of a thread-block cluster; the blocks sum their parts through distributed shared memory
 // in chunk order and each writes its share of the cell, so there are no partial images and the
@@ -368,7 +368,7 @@ __global__ void __launch_bounds__(kQueueThreads, 4)
 // R^k(c) once for the four partners (partner q adds to column R^(k+q)(c)): one 16-byte load and one
 // evaluation per four updates. Cells are 32 x 16 pixels of the quadrant.
 // Bound by issue at 14 warps per SM (1024 blocks). 512 x 512 pixels, 720 views of 768: 142 us one view at a
-// time, 92 us this way (2.05 T updates/s); the call 0.161 -> 0.114 ms.
+// time, 92 us this way (2.05 T updates/s); the call 0.161 -> 0.114 ms (0.104 with the filter's own scales).
 constexpr int kSymCellY = 16, kSymPairs = 2;
 
 // Indices of R^K of pixels (i, j): var along the thread's pixels, c the other one (Pixels).
