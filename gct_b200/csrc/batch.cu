@@ -163,7 +163,8 @@ std::string tune_key(const gct_fdk_plan *p, int num_sms)
     return std::to_string(p->device) + "/" + std::to_string(static_cast<int>(p->kind)) + "/" +
            std::to_string(p->opts.storage) + "/" + std::to_string(p->z_affine) + "/" + std::to_string(p->kx) +
            "x" + std::to_string(p->ky) + "x" + std::to_string(p->kz) + "/" + std::to_string(p->nr) + "x" +
-           std::to_string(p->nc) + "/" + std::to_string(num_sms) + "/q" + std::to_string(p->sym);
+           std::to_string(p->nc) + "/" + std::to_string(num_sms) + "/q" + std::to_string(p->sym) +
+           (p->rows ? "/rows" : "");  // the filter decides whether an FP16 line's stack is row pairs or quads
 }
 
 }  // namespace
