@@ -36,7 +36,8 @@ namespace {
 namespace cg = cooperative_groups;
 
 constexpr int kCell = 32;              // cell side in pixels
-constexpr int kThreads = 128;          // threads per cell: four warps side by side along x
+constexpr int kThreads = 128;          // threads of a group, which owns a cell: four warps side by side along x
+constexpr int kMaxGroups = 8;          // groups of a block: they share the block's views
 constexpr int kPairs = 4;              // pixel pairs per thread: pixels 4 apart along y
 constexpr int kStage = 32;             // views staged per barrier
 constexpr float kShift = 12582912.0f;  // 1.5 * 2^23: a sum with it holds a whole number in its low bits
@@ -49,7 +50,10 @@ struct CellView {
     float c0;
     int cls;
 };
-constexpr int kOff = 0, kInside = 1, kMixed = 2;  // the cell projects off the row, well inside it, or neither
+// The cell projects off the row, well inside it, or neither; kNear: neither, and near an arc's axis, where the
+// angle's polynomial holds (cells across the row's ends with atan2f: 257 x 257 pixels, 360 views 105 us a
+// call, 56 this way)
+constexpr int kOff = 0, kInside = 1, kMixed = 2, kNear = 3;
 
 // Where the thread's pixels are evaluated: at themselves, or in quarter-turn plans under the turns
 // that take the view to its base view. var: the index that varies over the thread's pixels (j; the
@@ -102,12 +106,13 @@ struct RowF16Partner : RowF16 {
     static constexpr unsigned kBytes = 16;
 };
 
-// Adds one view to the thread's pixels. INSIDE: the cell's samples lie well inside the row (and in
+// Adds one view to the thread's pixels. CLS kInside: the cell's samples lie well inside the row (and in
 // front of an arc's source, near its axis); else pixels that project off the row add nothing.
-template <int FAMILY, class R, bool ODD, bool INSIDE>
+template <int FAMILY, class R, bool ODD, int CLS>
 __device__ __forceinline__ void add_view(const CellView &v, const char *row, float umax, const Pixels &px,
                                          float2 (&acc)[kPairs])
 {
+    constexpr bool INSIDE = CLS == kInside;
     const float4 a = v.a, b = v.b;
     float v0[2] = {0.f, 0.f};
     if (FAMILY == 0) {  // rows j0 and j0 + 16, less the half of the centred split
@@ -133,7 +138,7 @@ __device__ __forceinline__ void add_view(const CellView &v, const char *row, flo
             } else {
                 const float2 rho2 = __ffma2_rn(u, u, __fmul2_rn(d, d));
                 w = __fmul2_rn(w, make_float2(rcp_approx(rho2.x), rcp_approx(rho2.y)));
-                const float2 g = INSIDE ? arc_angle_near(u, d) : make_float2(atan2f(u.x, d.x), atan2f(u.y, d.y));
+                const float2 g = CLS != kMixed ? arc_angle_near(u, d) : make_float2(atan2f(u.x, d.x), atan2f(u.y, d.y));
                 u = __ffma2_rn(g, two(b.w), two(v.c0));
             }
         }
@@ -193,14 +198,23 @@ __device__ void stage_view(const BpArgs &a, int v, int b, const Box &box, CellVi
     out.cls = !plain                                   ? kMixed
               : hi < -1.0f - m || lo > a.umax + m      ? kOff
               : lo >= -1.0f + m && hi <= a.umax - m    ? kInside
+              : FAMILY == 2                            ? kNear
                                                        : kMixed;
 }
 
-// Sums of views [a.v_begin, a.v_begin + a.v_count) for the 128 threads of the cell at pixel (i0, j0);
-// every thread of the block calls it (it holds block barriers), tid counts within the cell. SYM:
-// quarter-turn plans, whose views take their coordinates from the base view at the turned pixel.
-template <int FAMILY, class R, bool SYM>
-__device__ __forceinline__ void cell_sums(const BpArgs &a, int i0, int j0, int tid, CellView *s_view,
+// The 128 threads of a group wait for each other. GROUPS: the block has several (barrier 0 is the block's).
+template <bool GROUPS>
+__device__ __forceinline__ void group_sync(int group)
+{
+    if (GROUPS) asm volatile("bar.sync %0, %1;" ::"r"(group + 1), "n"(kThreads) : "memory");
+    else __syncthreads();
+}
+
+// Sums of views [a.v_begin, a.v_begin + a.v_count) over the cell at pixel (i0, j0) by one group of 128
+// threads (tid counts within it; all of them call it). SYM: quarter-turn plans, whose views take their
+// coordinates from the base view at the turned pixel.
+template <int FAMILY, class R, bool SYM, bool GROUPS>
+__device__ __forceinline__ void cell_sums(const BpArgs &a, int i0, int j0, int tid, int group, CellView *s_view,
                                           float2 (&acc)[kPairs])
 {
     const int lane = tid & 31;
@@ -245,41 +259,64 @@ __device__ __forceinline__ void cell_sums(const BpArgs &a, int i0, int j0, int t
         }
         for (; v < stop; v += kStage) {
             const int nvc = min(kStage, stop - v);
-            __syncthreads();
+            group_sync<GROUPS>(group);
             if (tid < nvc) stage_view<FAMILY>(a, v + tid, v + tid - q * (SYM ? a.quarter : 0), box, s_view[tid]);
-            __syncthreads();
+            group_sync<GROUPS>(group);
             const char *row = static_cast<const char *>(a.quads);
             if (R::kBytes == RowF16Partner::kBytes) row += static_cast<long long>(v - q * a.quarter) * row_bytes + 4 * q;
             else row += static_cast<long long>(v) * row_bytes;
             for (int k = 0; k < nvc; ++k, row += row_bytes) {
                 const int cls = s_view[k].cls;
                 if (cls == kOff) continue;  // every pixel of the cell would add zero
-                if (SYM && (q & 1)) {
-                    if (cls == kInside) add_view<FAMILY, R, true, true>(s_view[k], row, a.umax, px, acc);
-                    else add_view<FAMILY, R, true, false>(s_view[k], row, a.umax, px, acc);
-                } else {
-                    if (cls == kInside) add_view<FAMILY, R, false, true>(s_view[k], row, a.umax, px, acc);
-                    else add_view<FAMILY, R, false, false>(s_view[k], row, a.umax, px, acc);
-                }
+                auto add = [&](auto odd) {
+                    constexpr bool ODD = decltype(odd)::value;
+                    if (cls == kInside) add_view<FAMILY, R, ODD, kInside>(s_view[k], row, a.umax, px, acc);
+                    else if (FAMILY == 2 && cls == kNear) add_view<FAMILY, R, ODD, kNear>(s_view[k], row, a.umax, px, acc);
+                    else add_view<FAMILY, R, ODD, kMixed>(s_view[k], row, a.umax, px, acc);
+                };
+                if (SYM && (q & 1)) add(std::true_type());
+                else add(std::false_type());
             }
         }
         v = stop;
     }
 }
 
-// A cluster of gridDim.z blocks per cell, each with its chunk of the views.
-template <int FAMILY, class R, bool SYM>
-__global__ void __launch_bounds__(kThreads, 8) rows_kernel(BpArgs a, int chunk)
+// Shared memory of a group: its sums and its staged views.
+constexpr unsigned kRowsSmem = kCell * kCell * sizeof(float) + kStage * sizeof(CellView);
+
+// The block's sums [group][n] into [0], over the groups in order.
+__device__ __forceinline__ void sum_groups(float *s_sum, int n, int groups)
 {
-    __shared__ CellView s_view[kStage];
-    __shared__ float s_sum[kCell * kCell];  // [pixel][thread]: the block's sums
-    const int i0 = blockIdx.x * kCell, j0 = blockIdx.y * kCell, tid = threadIdx.x;
+    __syncthreads();
+    for (int e = threadIdx.x; e < n; e += blockDim.x) {
+        float s = s_sum[e];
+        for (int g = 1; g < groups; ++g) s += s_sum[g * n + e];
+        s_sum[e] = s;
+    }
+}
+
+// A cluster of gridDim.z blocks per cell, each with its chunk of the views; the groups of 128 threads of
+// a block share its chunk out among themselves.
+template <int FAMILY, class R, bool SYM, bool GROUPS>
+__global__ void __launch_bounds__(GROUPS ? kThreads * kMaxGroups : kThreads, GROUPS ? 1 : 8)
+    rows_kernel(BpArgs a, int chunk, int sub)
+{
+    extern __shared__ float4 s_mem[];  // GROUPS: kRowsSmem a group
+    __shared__ CellView s_view1[GROUPS ? 1 : kStage];
+    __shared__ float s_sum1[GROUPS ? 1 : kCell * kCell];
+    const int i0 = blockIdx.x * kCell, j0 = blockIdx.y * kCell, tid = GROUPS ? threadIdx.x % kThreads : threadIdx.x;
+    const int group = GROUPS ? threadIdx.x / kThreads : 0, groups = GROUPS ? blockDim.x / kThreads : 1;
+    float *const s_sum = GROUPS ? reinterpret_cast<float *>(s_mem) : s_sum1;  // [group][pixel][thread]
+    CellView *const s_view =
+        GROUPS ? reinterpret_cast<CellView *>(s_sum + groups * kCell * kCell) + group * kStage : s_view1;
     const int z = blockIdx.z, chunks = gridDim.z;
     BpArgs la = a;
-    la.v_begin = a.v_begin + z * chunk;
-    la.v_count = max(0, min(chunk, a.v_count - z * chunk));
+    const int first = z * chunk + group * sub, end = min((z + 1) * chunk, a.v_count);
+    la.v_begin = a.v_begin + first;
+    la.v_count = max(0, min(sub, end - first));
     float2 acc[kPairs];
-    cell_sums<FAMILY, R, SYM>(la, i0, j0, tid, s_view, acc);
+    cell_sums<FAMILY, R, SYM, GROUPS>(la, i0, j0, tid, group, s_view, acc);
     const int i = i0 + (tid >> 5) * 8 + (tid & 7), j = j0 + ((tid >> 3) & 3);
     auto put = [&](int p, float s) {
         const int y = j + 4 * p;
@@ -287,17 +324,19 @@ __global__ void __launch_bounds__(kThreads, 8) rows_kernel(BpArgs a, int chunk)
         float *dst = a.vol + static_cast<long long>(y) * a.nx + i;
         *dst = a.accumulate ? *dst + s : s;
     };
-    if (chunks == 1) {
+    if (chunks * groups == 1) {
 #pragma unroll
         for (int p = 0; p < 2 * kPairs; ++p) put(p, (p & 1) ? acc[p / 2].y : acc[p / 2].x);
         return;
     }
 #pragma unroll
-    for (int p = 0; p < 2 * kPairs; ++p) s_sum[p * kThreads + tid] = (p & 1) ? acc[p / 2].y : acc[p / 2].x;
+    for (int p = 0; p < 2 * kPairs; ++p)
+        s_sum[group * kCell * kCell + p * kThreads + tid] = (p & 1) ? acc[p / 2].y : acc[p / 2].x;
+    if (GROUPS) sum_groups(s_sum, kCell * kCell, groups);
     cg::cluster_group cl = cg::this_cluster();
     cl.sync();
-    // the block's share of the pixels (the chunks are 2, 4 or 8), over the chunks in order
-    for (int p = z; p < 2 * kPairs; p += chunks) {
+    // the block's share of the pixels (the chunks are 1, 2, 4 or 8), over the chunks in order
+    for (int p = z + chunks * group; p < 2 * kPairs; p += chunks * groups) {
         float s = 0.f;
         for (int c = 0; c < chunks; ++c) s += cl.map_shared_rank(s_sum, c)[p * kThreads + tid];
         put(p, s);
@@ -311,7 +350,7 @@ __device__ __noinline__ void queue_cells(const BpArgs &a, int tx, int ty, int ti
 {
     const int i0 = (2 * tx + tid / kThreads) * kCell, j0 = ty * kCell, ct = tid % kThreads;
     float2 acc[kPairs];
-    cell_sums<FAMILY, R, SYM>(a, i0, j0, ct, s_view + (tid / kThreads) * kStage, acc);
+    cell_sums<FAMILY, R, SYM, false>(a, i0, j0, ct, 0, s_view + (tid / kThreads) * kStage, acc);
     const int i = i0 + (ct >> 5) * 8 + (ct & 7), j = j0 + ((ct >> 3) & 3);
 #pragma unroll
     for (int p = 0; p < 2 * kPairs; ++p) {
@@ -369,7 +408,9 @@ __global__ void __launch_bounds__(kQueueThreads, 4)
 // evaluation per four updates. Cells are 32 x 16 pixels of the quadrant.
 // Bound by issue at 14 warps per SM (1024 blocks). 512 x 512 pixels, 720 views of 768: 142 us one view at a
 // time, 92 us this way (2.05 T updates/s); the call 0.161 -> 0.114 ms (0.104 with the filter's own scales).
-constexpr int kSymCellY = 16, kSymPairs = 2;
+constexpr int kSymCellY = 16, kSymPairs = 2, kSymGroups = 4;
+constexpr int kSymSums = 4 * 2 * kSymPairs * kThreads;  // a group's sums
+constexpr unsigned kSymSmem = kSymSums * sizeof(float) + kStage * (sizeof(float4) + sizeof(int4) + sizeof(CellView));
 
 // Indices of R^K of pixels (i, j): var along the thread's pixels, c the other one (Pixels).
 template <int K>
@@ -418,16 +459,24 @@ __device__ __forceinline__ void add_partners(const CellView &v, float4 w, const 
     }
 }
 
-// A cluster of gridDim.z blocks per cell, each with its chunk of the base views [a.v_begin, + a.v_count).
-__global__ void __launch_bounds__(kThreads, 6) rows_sym_kernel(BpArgs a, int chunk)
+// A cluster of gridDim.z blocks per cell, each with its chunk of the base views [a.v_begin, + a.v_count),
+// which the groups of a block share out among themselves.
+template <bool GROUPS>
+__global__ void __launch_bounds__(GROUPS ? kThreads * kSymGroups : kThreads, GROUPS ? 1 : 6)
+    rows_sym_kernel(BpArgs a, int chunk, int sub)
 {
-    __shared__ CellView s_view[kStage];
-    __shared__ float4 s_w[kStage];        // weight scales of the four partners
-    __shared__ int4 s_cls[kStage];        // class of the cell's four turned images
-    __shared__ float s_sum[4][2 * kSymPairs][kThreads];
-    const int i0 = blockIdx.x * kCell, j0 = blockIdx.y * kSymCellY, tid = threadIdx.x, h = a.nx / 2;
+    extern __shared__ float4 s_mem[];  // GROUPS: kSymSmem a group
+    __shared__ float4 s_mem1[GROUPS ? 1 : kSymSmem / sizeof(float4)];
+    const int tid = GROUPS ? threadIdx.x % kThreads : threadIdx.x;
+    const int group = GROUPS ? threadIdx.x / kThreads : 0, groups = GROUPS ? blockDim.x / kThreads : 1;
+    float *const s_sum = reinterpret_cast<float *>(GROUPS ? s_mem : s_mem1);  // [group][turn][pixel][thread]
+    float4 *const s_w = reinterpret_cast<float4 *>(s_sum + groups * kSymSums) + group * kStage;  // weights of the partners
+    int4 *const s_cls = reinterpret_cast<int4 *>(s_w + (groups - group) * kStage) + group * kStage;  // classes of the cell's turns
+    CellView *const s_view = reinterpret_cast<CellView *>(s_cls + (groups - group) * kStage) + group * kStage;
+    const int i0 = blockIdx.x * kCell, j0 = blockIdx.y * kSymCellY, h = a.nx / 2;
     const int z = blockIdx.z, chunks = gridDim.z;
-    const int v_begin = a.v_begin + z * chunk, v_end = min(v_begin + chunk, a.v_begin + a.v_count);
+    const int v_begin = a.v_begin + z * chunk + group * sub;
+    const int v_end = min(min(v_begin + sub, a.v_begin + (z + 1) * chunk), a.v_begin + a.v_count);
     const float n1 = static_cast<float>(a.nx - 1);
     const float i1 = static_cast<float>(min(i0 + kCell, h) - 1), j1 = static_cast<float>(min(j0 + kSymCellY, h) - 1);
     const int lane = tid & 31;
@@ -443,7 +492,7 @@ __global__ void __launch_bounds__(kThreads, 6) rows_sym_kernel(BpArgs a, int chu
     }
     for (int vc = v_begin; vc < v_end; vc += kStage) {
         const int nvc = min(kStage, v_end - vc);
-        __syncthreads();
+        group_sync<GROUPS>(group);
         if (tid / 4 < nvc) {
             const int sv = tid / 4, k = tid & 3, v = vc + sv;
             // the cell's box under k turns
@@ -458,7 +507,7 @@ __global__ void __launch_bounds__(kThreads, 6) rows_sym_kernel(BpArgs a, int chu
             reinterpret_cast<float *>(&s_w[sv])[k] = mine.a.w;
             if (k == 0) s_view[sv] = mine;
         }
-        __syncthreads();
+        group_sync<GROUPS>(group);
         const long long base_bytes = a.qview * 16;
         const char *row = static_cast<const char *>(a.quads) + vc * base_bytes;
         for (int k = 0; k < nvc; ++k, row += base_bytes) {
@@ -482,14 +531,16 @@ __global__ void __launch_bounds__(kThreads, 6) rows_sym_kernel(BpArgs a, int chu
 #pragma unroll
     for (int k = 0; k < 4; ++k)
 #pragma unroll
-        for (int p = 0; p < 2 * kSymPairs; ++p) s_sum[k][p][tid] = (p & 1) ? acc[k][p / 2].y : acc[k][p / 2].x;
+        for (int p = 0; p < 2 * kSymPairs; ++p)
+            s_sum[((group * 4 + k) * 2 * kSymPairs + p) * kThreads + tid] = (p & 1) ? acc[k][p / 2].y : acc[k][p / 2].x;
+    if (GROUPS) sum_groups(s_sum, kSymSums, groups);
     cg::cluster_group cl = cg::this_cluster();
     cl.sync();
     // the block's share of the pixels, over the chunks in order
-    for (int e = z; e < 8 * kSymPairs; e += chunks) {
+    for (int e = z + chunks * group; e < 8 * kSymPairs; e += chunks * groups) {
         const int k = e / (2 * kSymPairs), p = e % (2 * kSymPairs);
         float s = 0.f;
-        for (int c = 0; c < chunks; ++c) s += *cl.map_shared_rank(&s_sum[k][p][tid], c);
+        for (int c = 0; c < chunks; ++c) s += cl.map_shared_rank(s_sum, c)[e * kThreads + tid];
         int x = i0 + (tid >> 5) * 8 + (tid & 7), y = j0 + ((tid >> 3) & 3) + 4 * p;
         if (x >= h || y >= h) continue;
         for (int r = 0; r < k; ++r) {  // the plan's quarter turn
@@ -521,21 +572,34 @@ __global__ void row_pairs_kernel(const float *__restrict__ Y, int v0, int nv, in
     }
 }
 
-// Launches kern over clusters of view chunks per cell.
+// Launches kern over clusters of view chunks per cell; per_sm: its blocks that fit an SM. grouped: its form for
+// blocks of up to max_groups groups, with group_smem bytes of shared memory each.
 template <class Kern>
-void launch_cells(Kern kern, const BpArgs &a, dim3 cells, int num_sms, cudaStream_t s)
+void launch_cells(Kern kern, Kern grouped, const BpArgs &a, dim3 cells, int max_groups, int per_sm,
+                  unsigned group_smem, int num_sms, cudaStream_t s)
 {
     // chunks of at least 8 views until the grid holds six waves of eight blocks per SM: the last wave of
     // a launch of one to two waves runs nearly empty, and chunk counts that just fill whole waves measured
     // slower than finer ones (512 x 512 pixels one view at a time: 4 chunks 173 us, 8 chunks 142 us)
-    const long long want = 6LL * 8 * num_sms;
+    const long long n = static_cast<long long>(cells.x) * cells.y;
     int chunks = 1;
-    while (chunks < 8 && static_cast<long long>(cells.x) * cells.y * chunks < want && a.v_count / (2 * chunks) >= 8)
-        chunks *= 2;
+    while (chunks < 8 && n * chunks < 6LL * 8 * num_sms && a.v_count / (2 * chunks) >= 8) chunks *= 2;
     const int chunk = (a.v_count + chunks - 1) / chunks;
+    // An image of few cells leaves most of the SMs' warps idle with eight chunks, and a view costs a group
+    // its whole latency (0.6 us): then several groups share a chunk, as long as they fill at most half of the
+    // blocks that fit (between that and all of them the rest of the block waits for its slowest group:
+    // 257 x 254 pixels, 360 views, line 39.5 us as it is against 43.5 with two groups). Calls of 720
+    // views, F32: line 64 x 64 63 -> 25 us, 128 x 128 62 -> 29; arc, with the polynomial in kNear cells,
+    // 187 -> 32 and 187 -> 49 (the quad kernels' split launches took 36, 61, 40 and 78).
+    int groups = 1;
+    while (groups < max_groups && n * chunks * groups * 4 <= static_cast<long long>(per_sm) * num_sms &&
+           chunk / (2 * groups) >= 4)
+        groups *= 2;
+    const int sub = (chunk + groups - 1) / groups;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(cells.x, cells.y, chunks);
-    cfg.blockDim = dim3(kThreads);
+    cfg.blockDim = dim3(kThreads * groups);
+    cfg.dynamicSmemBytes = groups > 1 ? groups * group_smem : 0;
     cfg.stream = s;
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeClusterDimension;
@@ -544,21 +608,27 @@ void launch_cells(Kern kern, const BpArgs &a, dim3 cells, int num_sms, cudaStrea
     at[0].val.clusterDim.z = static_cast<unsigned>(chunks);
     cfg.attrs = at;
     cfg.numAttrs = 1;
-    cudaLaunchKernelEx(&cfg, kern, a, chunk);
+    cudaLaunchKernelEx(&cfg, groups > 1 ? grouped : kern, a, chunk, sub);
+}
+
+template <int FAMILY, class R, bool SYM>
+void launch_rows_kernel(const BpArgs &a, int num_sms, cudaStream_t s)
+{
+    launch_cells(rows_kernel<FAMILY, R, SYM, false>, rows_kernel<FAMILY, R, SYM, true>, a,
+                 dim3((a.nx + kCell - 1) / kCell, (a.ny + kCell - 1) / kCell), kMaxGroups, 8, kRowsSmem, num_sms, s);
 }
 
 template <class R>
 void launch_rows(const BpArgs &a, int family, int num_sms, cudaStream_t s)
 {
-    const dim3 cells((a.nx + kCell - 1) / kCell, (a.ny + kCell - 1) / kCell);
     if (family == 0) {
-        launch_cells(rows_kernel<0, R, false>, a, cells, num_sms, s);
+        launch_rows_kernel<0, R, false>(a, num_sms, s);
     } else if (family == 1) {
-        if (a.sym) launch_cells(rows_kernel<1, R, true>, a, cells, num_sms, s);
-        else launch_cells(rows_kernel<1, R, false>, a, cells, num_sms, s);
+        if (a.sym) launch_rows_kernel<1, R, true>(a, num_sms, s);
+        else launch_rows_kernel<1, R, false>(a, num_sms, s);
     } else if constexpr (R::kBytes == RowF32::kBytes) {
-        if (a.sym) launch_cells(rows_kernel<2, R, true>, a, cells, num_sms, s);
-        else launch_cells(rows_kernel<2, R, false>, a, cells, num_sms, s);
+        if (a.sym) launch_rows_kernel<2, R, true>(a, num_sms, s);
+        else launch_rows_kernel<2, R, false>(a, num_sms, s);
     }
 }
 
@@ -566,8 +636,7 @@ void launch_rows(const BpArgs &a, int family, int num_sms, cudaStream_t s)
 
 void launch_backproject_rows(const BpArgs &a, int family, int storage, int num_sms, cudaStream_t s)
 {
-    const dim3 cells((a.nx + kCell - 1) / kCell, (a.ny + kCell - 1) / kCell);
-    if (a.partners) launch_cells(rows_kernel<1, RowF16Partner, true>, a, cells, num_sms, s);
+    if (a.partners) launch_rows_kernel<1, RowF16Partner, true>(a, num_sms, s);
     else if (storage == 0) launch_rows<RowF32>(a, family, num_sms, s);
     else launch_rows<RowF16>(a, family, num_sms, s);
 }
@@ -575,7 +644,8 @@ void launch_backproject_rows(const BpArgs &a, int family, int storage, int num_s
 void launch_backproject_rows_sym(const BpArgs &a, int num_sms, cudaStream_t s)
 {
     const int h = a.nx / 2;
-    launch_cells(rows_sym_kernel, a, dim3((h + kCell - 1) / kCell, (h + kSymCellY - 1) / kSymCellY), num_sms, s);
+    launch_cells(rows_sym_kernel<false>, rows_sym_kernel<true>, a,
+                 dim3((h + kCell - 1) / kCell, (h + kSymCellY - 1) / kSymCellY), kSymGroups, 6, kSymSmem, num_sms, s);
 }
 
 int rows_queue_blocks_per_sm(int storage)
