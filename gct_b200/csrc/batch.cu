@@ -81,7 +81,7 @@ TileConfig default_config(const gct_fdk_plan *p, bool quarter_turn)
         c.zpt = vol3d(p) ? 8 : 1;
         c.bx = vol3d(p) ? 8 : 16;
         c.by = vol3d(p) ? 32 : 16;
-    } else if (p->rows) {  // rows.cu: 8 pixels per thread along y
+    } else if (p->rows) {  // rows.cu
         c.zpt = 1;
         c.bx = kRowsTileX;
         c.by = kQueueThreads / kRowsTileX;

@@ -161,7 +161,7 @@ inline bool queue_zpt_ok(int zpt) { return zpt == 1 || zpt == 4 || zpt == 8 || z
 // over row pairs.
 constexpr int kQueueClasses = 4;
 constexpr int kQueueSymClass = 2, kQueueRowsClass = 3;
-constexpr int kRowsTileX = 64, kRowsTileY = 32;  // pixels of a planar tile: two cells, 8 pixels per thread
+constexpr int kRowsTileX = 32, kRowsTileY = 32;  // pixels of a planar tile
 inline bool sym_queue_zpt_ok(int zpt) { return zpt == 1 || zpt == 8; }
 inline int queue_class(int zpt) { return zpt == 1 ? 0 : 1; }
 // Blocks of a queue kernel resident per SM for the storage type (0 f32, 1 f16) and depth class.

@@ -344,19 +344,28 @@ __global__ void __launch_bounds__(GROUPS ? kThreads * kMaxGroups : kThreads, GRO
     cl.sync();  // the sums stay until every block has read them
 }
 
-// Work-queue form: 256 threads take a tile of two cells side by side.
+// Work-queue form: the two groups of a block share the views of one cell. (One cell per group made a tile of
+// 64 x 32 pixels: a round with a single request, which the server must not split over the views in another
+// way than a full one, kept too few blocks busy. Line 512 x 512, 720 views, FP16, a request by itself: 0.90 ms, 0.62
+// with a cell per block; 48 at a time the same.)
 template <int FAMILY, class R, bool SYM>
-__device__ __noinline__ void queue_cells(const BpArgs &a, int tx, int ty, int tid, int mode, CellView *s_view)
+__device__ __noinline__ void queue_cell(BpArgs &a, int tx, int ty, int tid, int mode, CellView *s_view, float *s_sum)
 {
-    const int i0 = (2 * tx + tid / kThreads) * kCell, j0 = ty * kCell, ct = tid % kThreads;
+    const int i0 = tx * kCell, j0 = ty * kCell, group = tid / kThreads, ct = tid % kThreads;
     float2 acc[kPairs];
-    cell_sums<FAMILY, R, SYM, false>(a, i0, j0, ct, 0, s_view + (tid / kThreads) * kStage, acc);
+    cell_sums<FAMILY, R, SYM, true>(a, i0, j0, ct, group, s_view + group * kStage, acc);
+    // each group stores half of the pixels: its own sums of the others go through shared memory
+    const auto mine = [&](int p) { return (p & 1) ? acc[p / 2].y : acc[p / 2].x; };
+#pragma unroll
+    for (int p = 0; p < kPairs; ++p) s_sum[(group * kPairs + p) * kThreads + ct] = group ? mine(p) : mine(p + kPairs);
+    __syncthreads();
     const int i = i0 + (ct >> 5) * 8 + (ct & 7), j = j0 + ((ct >> 3) & 3);
 #pragma unroll
-    for (int p = 0; p < 2 * kPairs; ++p) {
-        const int y = j + 4 * p;
+    for (int p = 0; p < kPairs; ++p) {
+        const float other = s_sum[((1 - group) * kPairs + p) * kThreads + ct];
+        const float s = group ? other + mine(p + kPairs) : mine(p) + other;
+        const int y = j + 4 * (group * kPairs + p);
         if (i >= a.nx || y >= a.ny) continue;
-        const float s = (p & 1) ? acc[p / 2].y : acc[p / 2].x;
         float *dst = a.vol + static_cast<long long>(y) * a.nx + i;
         if (mode == kBpAtomic) atomicAdd(dst, s);
         else *dst = mode == kBpAccumulate ? *dst + s : s;
@@ -367,8 +376,9 @@ template <class R>
 __global__ void __launch_bounds__(kQueueThreads, 4)
     rows_queue_kernel(const BpItem *__restrict__ items, const BpWork *__restrict__ work, int n_work, int *counter)
 {
-    static_assert(kRowsTileX == (kQueueThreads / kThreads) * kCell && kRowsTileY == kCell, "tile of two cells");
-    __shared__ CellView s_view[kQueueThreads / kThreads * kStage];
+    static_assert(kQueueThreads == 2 * kThreads && kRowsTileX == kCell && kRowsTileY == kCell, "a cell of two groups");
+    __shared__ CellView s_view[2 * kStage];
+    __shared__ float s_sum[2 * kPairs * kThreads];
     __shared__ BpItem s_item;
     __shared__ BpWork s_work;
     __shared__ int s_next;
@@ -384,17 +394,18 @@ __global__ void __launch_bounds__(kQueueThreads, 4)
         }
         __syncthreads();
         BpArgs a = s_item.a;
-        a.v_begin = s_work.v_begin;
-        a.v_count = s_work.v_count;
+        const int count = tid < kThreads ? (s_work.v_count + 1) / 2 : s_work.v_count / 2;  // the first group takes the odd one
+        a.v_begin = s_work.v_begin + (tid < kThreads ? 0 : s_work.v_count - count);
+        a.v_count = count;
         const int mode = s_work.mode, tx = s_work.tile % s_item.tiles_x, ty = s_work.tile / s_item.tiles_x;
         if (s_item.family == 0) {
-            queue_cells<0, R, false>(a, tx, ty, tid, mode, s_view);
+            queue_cell<0, R, false>(a, tx, ty, tid, mode, s_view, s_sum);
         } else if (s_item.family == 1) {
-            if (a.sym) queue_cells<1, R, true>(a, tx, ty, tid, mode, s_view);
-            else queue_cells<1, R, false>(a, tx, ty, tid, mode, s_view);
+            if (a.sym) queue_cell<1, R, true>(a, tx, ty, tid, mode, s_view, s_sum);
+            else queue_cell<1, R, false>(a, tx, ty, tid, mode, s_view, s_sum);
         } else if constexpr (R::kBytes == RowF32::kBytes) {  // FP16 arcs keep their quads
-            if (a.sym) queue_cells<2, R, true>(a, tx, ty, tid, mode, s_view);
-            else queue_cells<2, R, false>(a, tx, ty, tid, mode, s_view);
+            if (a.sym) queue_cell<2, R, true>(a, tx, ty, tid, mode, s_view, s_sum);
+            else queue_cell<2, R, false>(a, tx, ty, tid, mode, s_view, s_sum);
         }
         __syncthreads();  // s_item / s_work / s_next are rewritten for the next entry
     }
@@ -589,7 +600,7 @@ void launch_cells(Kern kern, Kern grouped, const BpArgs &a, dim3 cells, int max_
     // its whole latency (0.6 us): then several groups share a chunk, as long as they fill at most half of the
     // blocks that fit (between that and all of them the rest of the block waits for its slowest group:
     // 257 x 254 pixels, 360 views, line 39.5 us as it is against 43.5 with two groups). Calls of 720
-    // views, F32: line 64 x 64 63 -> 25 us, 128 x 128 62 -> 29; arc, with the polynomial in kNear cells,
+    // views, F32: line 64 x 64 63 -> 25 us, 128 x 128 62 -> 33; arc, with the polynomial in kNear cells,
     // 187 -> 32 and 187 -> 49 (the quad kernels' split launches took 36, 61, 40 and 78).
     int groups = 1;
     while (groups < max_groups && n * chunks * groups * 4 <= static_cast<long long>(per_sm) * num_sms &&
