@@ -95,6 +95,47 @@ void toeplitz_f16(gct_fdk_plan *p, const std::vector<double> &taps, std::vector<
     }
 }
 
+// Slices per thread of a spiral scan's z-affine backprojection (1, 4 or 8) from the slices' view windows
+// (first, count). A thread walks the union of its slices' windows. Per view of it, four slices cost a full
+// device 1.45 and eight 2.15 times what one slice costs (FP32), however many of them take the view, so depth
+// pays where neighbouring windows overlap; and the fewer, deeper threads of a small volume wait out a view's
+// latency, which grows with the depth too and is as long as a full device takes over some 500 columns per SM. The
+// numbers below are fitted to the times of 244 forms (both detectors and storages, 32 to 512 columns a side,
+// windows 4 to 540 views apart) under the condition that none gets slower than with one slice. Cylindrical, 360 views a turn,
+// FP32, one / four / eight slices per thread: 512 x 512 x 24, windows 4 views apart 8.0 / 3.1 / 2.3 ms, 90 apart
+// 8.0 / 5.1 / 5.6; 256 x 256 x 24, 180 apart 2.08 / 2.24 / 2.89; 64 x 64 x 64, 4 apart 0.39 / 0.22 / 0.32; 32 x 32 x 64,
+// 12 apart 0.16 / 0.21 / 0.39. Always eight lost up to half of the speed of one; the choice is 1 % slower than the
+// best of the three on average.
+int spiral_depth(const std::vector<int2> &win, double columns, bool f16, int num_sms)
+{
+    const int depth[3] = {1, 4, 8};
+    const double cost[3] = {1.0, f16 ? 1.4 : 1.65, f16 ? 1.9 : 2.4}, latency[3] = {1.0, 1.35, 2.1};
+    int best = 1;
+    double best_t = 0.0;
+    for (int d = 0; d < 3; ++d) {
+        double total = 0.0, longest = 0.0;
+        for (size_t k = 0; k < win.size(); k += depth[d]) {
+            std::vector<int2> w(win.begin() + k, win.begin() + std::min(win.size(), k + depth[d]));
+            std::sort(w.begin(), w.end(), [](const int2 &a, const int2 &b) { return a.x < b.x; });
+            double views = 0.0;
+            int end = 0;
+            for (const int2 &v : w) {
+                views += std::max(0, v.x + v.y - std::max(end, v.x));
+                end = std::max(end, v.x + v.y);
+            }
+            total += views;
+            longest = std::max(longest, views);
+        }
+        double t = std::hypot(cost[d] * columns * total, latency[d] * (f16 ? 600.0 : 500.0) * num_sms * longest);
+        if (d == 0) t *= 0.75;  // depth has to be worth a quarter, more than the model is off
+        if (d == 0 || t < best_t) {
+            best_t = t;
+            best = depth[d];
+        }
+    }
+    return best;
+}
+
 void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
                 const gct_filt_params *filt, const gct_fdk_opts *opts)
 {
@@ -290,13 +331,7 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
     if (p->sym && !p->rows && !p->ybuf.p)
         p->ybuf.alloc(static_cast<size_t>(p->nv) * p->nr * p->nc, "filtered rows of quarter-turn stacks");
     if (p->spiral) {
-        // each slice has its own window of views: z-affine geometries take several slices per thread
-        // over the union of their windows, others one
         p->sym = 0;
-        if (p->opts.z_per_thread <= 0) p->zpt = 8;
-        if (!p->z_affine || p->zpt < 4) p->zpt = 1;
-        if (p->opts.block_x <= 0) p->bx = f16 ? 8 : 4;
-        if (p->opts.block_y <= 0) p->by = 16;
         std::vector<int2> win(p->kz);
         const double z0 = vol->mid[2] - (vol->nz - 1.0) * vol->dz / 2.0;
         for (int k = 0; k < p->kz; ++k) {
@@ -305,6 +340,12 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
             win[k] = (first > 0 && last < p->nv) ? make_int2(static_cast<int>(first), static_cast<int>(last - first))
                                                  : make_int2(0, 0);
         }
+        // z-affine geometries take several slices per thread over the union of their windows, others one
+        if (p->opts.z_per_thread <= 0) p->zpt = spiral_depth(win, static_cast<double>(p->kx) * p->ky, f16, p->num_sms);
+        if (!p->z_affine || p->zpt < 4) p->zpt = 1;
+        // one slice per thread: 32 x 8 (flat 512 x 512 x 24, 360 views a turn: 6.2 ms against 6.4 with 4 x 16)
+        if (p->opts.block_x <= 0) p->bx = p->zpt == 1 ? 32 : f16 ? 8 : 4;
+        if (p->opts.block_y <= 0) p->by = p->zpt == 1 ? 8 : 16;
         p->slice_views.upload(win.data(), win.size(), "spiral slice windows");
     }
     p->zpt_sym = p->opts.z_per_thread > 0 ? std::min(p->zpt, 8) : (vol3d ? (f16 ? 8 : 4) : 1);

@@ -481,7 +481,7 @@ __global__ void __launch_bounds__(256) bp_kernel(BpArgs a)
 // paid for the arc's angle and the projection again: 96 x 256 x 256 voxels, 576 views a turn, 64 x 448
 // detector (3.6e9 updates), FP32: 10.5 ms, 8.8 ms with the arc angle as a polynomial, 4.0 ms with eight
 // slices (four 4.4, sixteen 5.6: the union of their windows grows; 8 x 16 and 8 x 8 blocks within 1 %, 32 x 8
-// 4.5).
+// 4.5). Where windows overlap less, or columns are few, fewer slices per thread are faster (spiral_depth, abi.cu).
 template <int FAMILY, class Q, int ZPT>
 __global__ void __launch_bounds__(256) bp_spiral_kernel(BpArgs a)
 {
@@ -536,9 +536,7 @@ __global__ void __launch_bounds__(256) bp_spiral_kernel(BpArgs a)
                     column_dispatch<L, ZPT, false, true>(view, 1, a.qpitch, u, v0, vs, a.umax, a.vmax, wt, acc,
                                                          kBoxMixed, nullptr, on);
             };
-            if (FAMILY == 0) {
-                add(fmaf(c[2], fj, fmaf(c[1], fi, c[0])), fmaf(c[4], fk0, c[3]), c[4], ConstWeight{ws});
-            } else if (FAMILY == 1) {
+            if (FAMILY == 1) {
                 const float inv = rcp_approx(fmaf(c[10], fj, fmaf(c[9], fi, c[8])));
                 add(fmaf(c[2], fj, fmaf(c[1], fi, c[0])) * inv,
                     fmaf(c[7], fk0, fmaf(c[6], fj, fmaf(c[5], fi, c[4]))) * inv, c[7] * inv, ConstWeight{ws * inv * inv});
@@ -588,8 +586,8 @@ void launch_zpt(const BpArgs &a, bool z_affine, dim3 grid, dim3 block, cudaStrea
             return;
         }
     }
-    if constexpr (ZPT == 4 || ZPT == 8 || ZPT == 16) {
-        if (a.slice_views) {  // one slice per thread where the geometry is not z-affine
+    if constexpr (FAMILY != 0 && (ZPT == 4 || ZPT == 8 || ZPT == 16)) {
+        if (a.slice_views) {  // one slice per thread where the geometry is not z-affine (spirals are cone beams)
             bp_spiral_kernel<FAMILY, Q, ZPT><<<grid, block, 0, s>>>(a);
             return;
         }

@@ -88,8 +88,8 @@ struct BpArgs {
     int accumulate = 0;
     int quarter = 0;  // quad_layout of the stack
     int partners = 0;  // row pairs: interleaved partner views (FP16 lines)
-    // spiral scans (one voxel per thread along z): slice k backprojects views [x, x + y) of
-    // slice_views[k], intersected with [v_begin, v_begin + v_count)
+    // spiral scans: slice k backprojects views [x, x + y) of slice_views[k], intersected with
+    // [v_begin, v_begin + v_count)
     const int2 *slice_views = nullptr;
     // quarter-turn launches (quarter > 0): v_begin / v_count count base views, whose partners are
     // v + q * quarter (q = 1..3); sym (+1 / -1) is the turn that maps their voxel columns
