@@ -279,7 +279,7 @@ template <class L>
 __device__ __forceinline__ float ray_angle(float A, float B)
 {
     if (std::is_same<L, LerpF32>::value && B > 0.f && fabsf(A) <= kArcNear * B)
-        return arc_angle_near(make_float2(A, A), make_float2(B, B)).x;
+        return -arc_angle_near_neg(make_float2(A, A), make_float2(B, B)).x;
     return atan2f(A, B);
 }
 

@@ -132,16 +132,18 @@ __device__ __forceinline__ float rcp_approx(float x)
     return r;
 }
 
-// atan2(A, B) for B > 0, |A| <= kArcNear B: the quotient t with one correction step, then t + t s Q(s),
-// s = t^2, Q the polynomial of degree 6 fitted to (atan(t) / t - 1) / s by least squares at 200 Chebyshev
-// nodes of s in [0, 9/16] (relative error 1.6e-8 with these FP32 coefficients).
+// -atan2(A, B) for B > 0, |A| <= kArcNear B (negated: the reciprocal of -B saves the sign changes): with the
+// approximate quotient t and what it is short of, t' = (A - t B) / B, the angle is t + (t s Q(s) + t'), s = t^2, Q
+// the polynomial of degree 6 fitted to (atan(t) / t - 1) / s by least squares at 200 Chebyshev nodes of s in
+// [0, 9/16] (relative error 1.6e-8 with these FP32 coefficients). One rounding at the angle's size: over 4e6 pairs
+// its rms error is 0.31 units in the last place, atan2f's 0.39 (0.39 too with t + t' rounded first).
 constexpr float kArcNear = 0.75f;
-__device__ __forceinline__ float2 arc_angle_near(float2 A, float2 B)
+__device__ __forceinline__ float2 arc_angle_near_neg(float2 A, float2 B)
 {
-    const float2 inv = make_float2(rcp_approx(B.x), rcp_approx(B.y));
+    const float2 inv = make_float2(rcp_approx(-B.x), rcp_approx(-B.y));
     const auto two = [](float x) { return make_float2(x, x); };
-    float2 t = __fmul2_rn(A, inv);
-    t = __ffma2_rn(__ffma2_rn(__fmul2_rn(t, two(-1.f)), B, A), inv, t);
+    const float2 t = __fmul2_rn(A, inv);
+    const float2 low = __fmul2_rn(__ffma2_rn(t, B, A), inv);
     const float2 s = __fmul2_rn(t, t);
     float2 q = __ffma2_rn(s, two(-0.0155409574508667f), two(0.04879451543092728f));
     q = __ffma2_rn(q, s, two(-0.08184777945280075f));
@@ -149,7 +151,7 @@ __device__ __forceinline__ float2 arc_angle_near(float2 A, float2 B)
     q = __ffma2_rn(q, s, two(-0.1427159309387207f));
     q = __ffma2_rn(q, s, two(0.1999952644109726f));
     q = __ffma2_rn(q, s, two(-0.3333333134651184f));
-    return __ffma2_rn(__fmul2_rn(t, s), q, t);
+    return __fadd2_rn(t, __ffma2_rn(__fmul2_rn(t, s), q, low));
 }
 
 }  // namespace gct

@@ -44,7 +44,7 @@ constexpr float kShift = 12582912.0f;  // 1.5 * 2^23: a sum with it holds a whol
 constexpr unsigned kShiftBits = 0x4B400000u;
 
 // One view of a cell: a = first form (u, U or A) at pixel (0, 0), per i and j step, and the weight
-// scale; b = second form (D or B) and 1 / dgamma; c0 = column of an arc's central ray.
+// scale; b = second form (D or B) and -1 / dgamma; c0 = column of an arc's central ray.
 struct CellView {
     float4 a, b;
     float c0;
@@ -52,7 +52,7 @@ struct CellView {
 };
 // The cell projects off the row, well inside it, or neither; kNear: neither, and near an arc's axis, where the
 // angle's polynomial holds (cells across the row's ends with atan2f: 257 x 257 pixels, 360 views 105 us a
-// call, 56 this way)
+// call, 68 this way)
 constexpr int kOff = 0, kInside = 1, kMixed = 2, kNear = 3;
 
 // Where the thread's pixels are evaluated: at themselves, or in quarter-turn plans under the turns
@@ -106,13 +106,12 @@ struct RowF16Partner : RowF16 {
     static constexpr unsigned kBytes = 16;
 };
 
-// Adds one view to the thread's pixels. CLS kInside: the cell's samples lie well inside the row (and in
+// Adds one view to the thread's pixels. INSIDE: the cell's samples lie well inside the row (and in
 // front of an arc's source, near its axis); else pixels that project off the row add nothing.
-template <int FAMILY, class R, bool ODD, int CLS>
+template <int FAMILY, class R, bool ODD, bool INSIDE>
 __device__ __forceinline__ void add_view(const CellView &v, const char *row, float umax, const Pixels &px,
                                          float2 (&acc)[kPairs])
 {
-    constexpr bool INSIDE = CLS == kInside;
     const float4 a = v.a, b = v.b;
     float v0[2] = {0.f, 0.f};
     if (FAMILY == 0) {  // rows j0 and j0 + 16, less the half of the centred split
@@ -138,7 +137,8 @@ __device__ __forceinline__ void add_view(const CellView &v, const char *row, flo
             } else {
                 const float2 rho2 = __ffma2_rn(u, u, __fmul2_rn(d, d));
                 w = __fmul2_rn(w, make_float2(rcp_approx(rho2.x), rcp_approx(rho2.y)));
-                const float2 g = CLS != kMixed ? arc_angle_near(u, d) : make_float2(atan2f(u.x, d.x), atan2f(u.y, d.y));
+                const float2 g = INSIDE || v.cls == kNear ? arc_angle_near_neg(u, d)
+                                                          : make_float2(-atan2f(u.x, d.x), -atan2f(u.y, d.y));
                 u = __ffma2_rn(g, two(b.w), two(v.c0));
             }
         }
@@ -161,6 +161,19 @@ __device__ __forceinline__ void add_view(const CellView &v, const char *row, flo
     }
 }
 
+// add_view for an arc's kNear and kMixed views as a call: in line they take registers and instruction
+// cache from the kInside views, most of them (509 x 387 pixels, 1151 views: 267 us with atan2f for both, 275
+// with the kNear form, both in line, 263 this way).
+struct Sums {
+    float2 s[kPairs];
+};
+template <class R, bool ODD>
+__device__ __noinline__ Sums add_edge_view(CellView v, const char *row, float umax, Pixels px, Sums sums)
+{
+    add_view<2, R, ODD, false>(v, row, umax, px, sums.s);
+    return sums;
+}
+
 // Index box of a cell's pixels in the image.
 struct Box {
     float i0, i1, j0, j1;
@@ -178,7 +191,7 @@ __device__ void stage_view(const BpArgs &a, int v, int b, const Box &box, CellVi
     if (a.vinv) w *= __ldg(a.vinv + v);
     out.a = make_float4(__ldg(c), __ldg(c + 1), __ldg(c + 2), w);
     out.b = FAMILY == 0 ? make_float4(0.f, 0.f, 0.f, 0.f)
-                        : make_float4(__ldg(c + kD), __ldg(c + kD + 1), __ldg(c + kD + 2), __ldg(c + 12));
+                        : make_float4(__ldg(c + kD), __ldg(c + kD + 1), __ldg(c + kD + 2), FAMILY == 2 ? -__ldg(c + 12) : 0.f);
     out.c0 = FAMILY == 2 ? __ldg(c + 13) : 0.f;
     float lo = 3.0e38f, hi = -3.0e38f;
     bool plain = true;
@@ -189,7 +202,7 @@ __device__ void stage_view(const BpArgs &a, int v, int b, const Box &box, CellVi
         if (FAMILY != 0) {
             const float d = fmaf(out.b.z, j, fmaf(out.b.y, i, out.b.x));
             if (!(d > 0.f) || (FAMILY == 2 && !(fabsf(u) <= kArcNear * d))) plain = false;
-            u = FAMILY == 1 ? u / d : fmaf(atan2f(u, d), out.b.w, out.c0);
+            u = FAMILY == 1 ? u / d : fmaf(-atan2f(u, d), out.b.w, out.c0);
         }
         lo = fminf(lo, u);
         hi = fmaxf(hi, u);
@@ -270,9 +283,18 @@ __device__ __forceinline__ void cell_sums(const BpArgs &a, int i0, int j0, int t
                 if (cls == kOff) continue;  // every pixel of the cell would add zero
                 auto add = [&](auto odd) {
                     constexpr bool ODD = decltype(odd)::value;
-                    if (cls == kInside) add_view<FAMILY, R, ODD, kInside>(s_view[k], row, a.umax, px, acc);
-                    else if (FAMILY == 2 && cls == kNear) add_view<FAMILY, R, ODD, kNear>(s_view[k], row, a.umax, px, acc);
-                    else add_view<FAMILY, R, ODD, kMixed>(s_view[k], row, a.umax, px, acc);
+                    if (cls == kInside) {
+                        add_view<FAMILY, R, ODD, true>(s_view[k], row, a.umax, px, acc);
+                    } else if constexpr (FAMILY == 2) {
+                        Sums t;
+#pragma unroll
+                        for (int p = 0; p < kPairs; ++p) t.s[p] = acc[p];
+                        t = add_edge_view<R, ODD>(s_view[k], row, a.umax, px, t);
+#pragma unroll
+                        for (int p = 0; p < kPairs; ++p) acc[p] = t.s[p];
+                    } else {
+                        add_view<FAMILY, R, ODD, false>(s_view[k], row, a.umax, px, acc);
+                    }
                 };
                 if (SYM && (q & 1)) add(std::true_type());
                 else add(std::false_type());
@@ -600,8 +622,8 @@ void launch_cells(Kern kern, Kern grouped, const BpArgs &a, dim3 cells, int max_
     // its whole latency (0.6 us): then several groups share a chunk, as long as they fill at most half of the
     // blocks that fit (between that and all of them the rest of the block waits for its slowest group:
     // 257 x 254 pixels, 360 views, line 39.5 us as it is against 43.5 with two groups). Calls of 720
-    // views, F32: line 64 x 64 63 -> 25 us, 128 x 128 62 -> 33; arc, with the polynomial in kNear cells,
-    // 187 -> 32 and 187 -> 49 (the quad kernels' split launches took 36, 61, 40 and 78).
+    // views, F32: line 64 x 64 68 -> 25 us, 128 x 128 63 -> 32; arc, with the polynomial in kNear cells,
+    // 194 -> 36 and 189 -> 52 (the quad kernels' split launches took 35, 60, 40 and 77).
     int groups = 1;
     while (groups < max_groups && n * chunks * groups * 4 <= static_cast<long long>(per_sm) * num_sms &&
            chunk / (2 * groups) >= 4)
