@@ -289,20 +289,31 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
     const bool f16 = p->opts.storage == GCT_STORAGE_F16;
     // row-pair plans have a fixed shape of their own (rows.cu); their options are checked all the same
     const bool par1d = kind == GCT_GEOM_PARALLEL_1D;
-    // FP32 quads, 4 x 16 blocks: 8 voxels per thread for the parallel kinds (256 x 256 x 160 / 300 views: 2.84
-    // against 3.79 ms) and for flat panels over at most 256 x 256 columns (256^3 / 360 views 4.30 against
-    // 4.40, short scan 253 x 241 x 187 2.82 against 2.95); larger grids lose (381 x 381 x 290 / 500 views 16.9
-    // against 16.0, 512^3 72.1 against 70.2), and so do arcs (381 x 379 x 61 / 577 views 5.6 against 5.4)
-    const bool shallow = !f16 && (p->family == gct::Family::Affine ||
-                                  (p->family == gct::Family::Projective && p->z_affine &&
-                                   static_cast<long long>(p->kx) * p->ky <= 256 * 256));
-    p->zpt = p->opts.z_per_thread > 0 ? p->opts.z_per_thread : vol3d ? (shallow ? 8 : 16) : 1;
-    if (p->zpt != 1 && p->zpt != 2 && p->zpt != 4 && p->zpt != 8 && p->zpt != 16)
+    const int zo = p->opts.z_per_thread;
+    if (zo > 0 && zo != 1 && zo != 2 && zo != 4 && zo != 8 && zo != 16)
         gct::fail(GCT_ERR_INVALID_ARG, "z_per_thread must be 1, 2, 4, 8 or 16");
     p->bx = p->opts.block_x > 0 ? p->opts.block_x : (par1d ? 128 : vol3d ? (f16 ? 8 : 4) : 32);
     p->by = p->opts.block_y > 0 ? p->opts.block_y : (par1d ? 1 : vol3d ? 16 : 8);
     if (p->bx * p->by > 256 || p->bx * p->by < 32)
         gct::fail(GCT_ERR_INVALID_ARG, "backprojection block must hold 32..256 threads");
+    // FP32 quads of the parallel kinds: 8 voxels per thread (240 views: 64 x 64 x 32 0.18 against 0.40 ms with 16,
+    // 256 x 256 x 256 3.5 against 4.2, 512 x 512 x 256 11.8 against 12.8).
+    // Of flat panels: a wave of blocks with 16 voxels (16 blocks of 64 threads per SM) takes 1.9 times as long
+    // as one with 8 (465 and 245 us with 240 views), so 8 where the last wave of 16 leaves more than that
+    // empty. 240 views: 128 x 128 x 32 0.21 (8) against 0.35 ms (16), 224 x 224 x 56 0.73 against 0.83, 320 x 320 x 80 1.62
+    // against 1.81, 253 x 241 x 187 (short scan, 247 views) 2.85 against 2.96; the other way 192^3 1.60 against 1.42,
+    // 256^3 3.47 against 3.23, 512^3 27.2 against 25.8.
+    // Arcs keep 16 (381 x 379 x 61, 577 views 5.4 ms, 5.6 with 8).
+    const auto waves = [&](int z) {
+        const long long blocks = static_cast<long long>((p->kx + p->bx - 1) / p->bx) *
+                                 ((p->ky + p->by - 1) / p->by) * ((p->kz + z - 1) / z);
+        const long long wave = 1024LL / (p->bx * p->by) * p->num_sms;
+        return static_cast<double>((blocks + wave - 1) / wave);
+    };
+    const bool shallow = !f16 && vol3d &&
+                         (p->family == gct::Family::Affine ||
+                          (p->family == gct::Family::Projective && p->z_affine && waves(8) < 1.9 * waves(16)));
+    p->zpt = zo > 0 ? zo : vol3d ? (shallow ? 8 : 16) : 1;
     // quarter-turn form: the z-affine column kernels and the fans over row pairs (not the 1D parallel
     // kind); at most 8 voxels per thread, since each thread keeps four columns.
     // Measured on B200 (512^3, 720 views): FP16 quads 34.4 ms against 47.2 ms for the plain kernel
