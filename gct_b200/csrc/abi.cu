@@ -1447,16 +1447,26 @@ gct_status gct_forward_project(const gct_ct_geom *geom, const gct_vol_geom *vol,
         cudaGetDevice(&dev);
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev);
         const int nr = vol3d ? static_cast<int>(geom->det_col.num_samples) : 1;
-        // the copies of the grid that the rays read; without memory for them the grid is read as it is
-        DevBuf<float> copies;
-        try {
-            copies.alloc(static_cast<size_t>(gct::forward_scratch_floats(box)), "grid copies");
-        } catch (const gct::GctError &) {
+        const int nv = static_cast<int>(geom->num_views), nc = static_cast<int>(geom->det_row.num_samples);
+        // the copies of the grid that the rays read; they leave others half of the free memory, and without
+        // memory for them the grid is read as it is
+        gct::ForwardCopies copies = gct::forward_copies(box, pv.data(), kind, nv, nr, nc, step_vox);
+        const size_t floats = static_cast<size_t>(gct::forward_copy_floats(box, copies));
+        if (floats * sizeof(float) > (size_t{1} << 30)) {
+            size_t free_b = 0, total_b = 0;
+            cuda_check(cudaMemGetInfo(&free_b, &total_b), "cudaMemGetInfo");
+            if (floats * sizeof(float) > free_b / 2) copies = gct::ForwardCopies::None;
         }
-        gct::launch_forward(dv.p, kind, static_cast<int>(geom->num_views), nr,
-                            static_cast<int>(geom->det_row.num_samples), geom->det_row.sampling_width,
-                            vol3d ? geom->det_col.sampling_width : 1.0, vol_dev, copies.p, box, step_vox, proj_dev, sms,
-                            s);
+        DevBuf<float> scratch;
+        try {
+            if (copies != gct::ForwardCopies::None) scratch.alloc(floats, "grid copies");
+        } catch (const gct::GctError &e) {
+            if (e.status != GCT_ERR_OUT_OF_MEMORY) throw;
+            copies = gct::ForwardCopies::None;
+        }
+        gct::launch_forward(dv.p, kind, nv, nr, nc, geom->det_row.sampling_width,
+                            vol3d ? geom->det_col.sampling_width : 1.0, vol_dev, copies, scratch.p, box, step_vox,
+                            proj_dev, sms, s);
         cuda_check(cudaGetLastError(), "forward projector launch");
         cuda_check(cudaStreamSynchronize(s), "forward projection");
     });

@@ -7,7 +7,9 @@
 //   arc / cylinder : origin S, direction cos(g) e_w + sin(g) e_u + (t / SDD) e_v
 // with u = (c - c0) du, v = (r - r0) dv (src/cuda/geom/coord_trans_proj.cuh:142-150, the
 // inverse of DCSToPCS).
+#include <algorithm>
 #include <climits>
+#include <cmath>
 
 #include "../../include/gct_fdk.h"
 #include "project.hpp"
@@ -19,6 +21,17 @@ namespace {
 // the copies than the copies save (25 x 25 x 24 voxels, 36 views of 48 x 40: 0.69 ms a call against
 // 0.75 with copies; 32 x 32 x 31, 90 views of 64 x 64: 0.75 against 0.84).
 constexpr long long kCopyVoxels = 1 << 14;
+// What copies cost a call and save it, in us. Up to 2 MB they come with the driver's smallest allocations and
+// cost next to nothing (48^3 voxels, 4 views of 64 x 64 and more: 0 to 15 % less time with them); larger ones cost
+// 0.5 ms and 18 us per million voxels, the exchanged grid alone 5 us. A million samples of rays along x, within
+// the tenth of a voxel of y per step that keeps the warp from marching in step, take 15 to 24 us longer in the
+// grid itself than in either copy (every gather touches 32 lines); others
+// take 0.8 us longer than in the pairs. Without / exchanged grid / pairs, ms a call: 2 views of 64 x 64 through 512^3
+// 1.4 / - / 4.9, of 256 x 256 5.0 / 3.3 / 5.2, of 512 x 512 10.4 / 3.4 / 5.8; 8 views of 96 x 96 through 96^3 1.0 / - / 1.4,
+// 180 of 160 x 160 5.3 / - / 3.3; 192^3, 16 views of 256 x 256, half-voxel steps 2.7 / - / 2.3, whole ones 1.8 / - / 2.0.
+constexpr long long kSmallCopies = 2 << 20;
+constexpr double kCopyCall = 500.0, kPairsVoxel = 18e-6, kAlongVoxel = 5e-6;
+constexpr double kSaveX = 21e-6, kPairsSave = 0.8e-6;
 
 struct Ray {
     double o[3];
@@ -245,7 +258,9 @@ __device__ __forceinline__ float forward_ray(const Ray &ray, bool on, const floa
     auto at2 = [](const char *row, Off o) { return __ldg(reinterpret_cast<const float2 *>(row + o)); };
     float2 sum2 = make_float2(0.f, 0.f);
     for (int k0 = __reduce_min_sync(0xffffffffu, ka); k0 < kend; k0 += kChunk) {
-        if (ka >= k0 + kChunk || kb <= k0) continue;  // no sample of this lane in the chunk
+        const bool here = ka < k0 + kChunk && kb > k0;  // else no sample of this lane in the chunk
+        const unsigned lanes = __ballot_sync(0xffffffffu, here);
+        if (!here) continue;
         float r[3] = {0.f, 0.f, 0.f};
         long long c[3] = {0, 0, 0};
 #pragma unroll
@@ -293,14 +308,18 @@ __device__ __forceinline__ float forward_ray(const Ray &ray, bool on, const floa
                              g[NA - 1]);
             }
         };
-        const float lo = static_cast<float>(max(ka - k0, 0)), hi = static_cast<float>(min(kb - k0, kChunk) - 1);
-        float2 fk = make_float2(0.f, 1.f);
-        if (__all_sync(__activemask(), lo == 0.f && hi == kChunk - 1.f)) {
+        const int first = max(ka - k0, 0), last = min(kb - k0, kChunk) - 1;
+        if (__all_sync(lanes, first == 0 && last == kChunk - 1)) {
+            float2 fk = make_float2(0.f, 1.f);
 #pragma unroll 1
             for (int k = 0; k < kChunk; k += 2, fk = __fadd2_rn(fk, make_float2(2.f, 2.f))) sum2 = __fadd2_rn(sum2, pair(fk));
         } else {  // some ray starts or ends in the chunk: its other samples repeat its first or last one, unsummed
+            const float lo = static_cast<float>(first), hi = static_cast<float>(last);
+            const int k1 = __reduce_max_sync(lanes, last);
+            int k = __reduce_min_sync(lanes, first);
+            float2 fk = make_float2(static_cast<float>(k), static_cast<float>(k + 1));
 #pragma unroll 1
-            for (int k = 0; k < kChunk; k += 2, fk = __fadd2_rn(fk, make_float2(2.f, 2.f))) {
+            for (; k <= k1; k += 2, fk = __fadd2_rn(fk, make_float2(2.f, 2.f))) {
                 const float2 fc = make_float2(fminf(fmaxf(fk.x, lo), hi), fminf(fmaxf(fk.y, lo), hi));
                 const float2 e = pair(fc);
                 sum2.x += fc.x == fk.x ? e.x : 0.f;
@@ -417,20 +436,21 @@ void launch_phantom(const ProjView *views, int kind, int nv, int nr, int nc, dou
 }
 
 void launch_forward(const ProjView *views, int kind, int nv, int nr, int nc, double du, double dv,
-                    const float *vol, float *scratch, const VolBox &box, float step_vox, float *out, int num_sms,
-                    cudaStream_t s)
+                    const float *vol, ForwardCopies copies, float *scratch, const VolBox &box, float step_vox, float *out,
+                    int num_sms, cudaStream_t s)
 {
     const long long voxels = static_cast<long long>(box.nx) * box.ny * box.nz;
     const float *across = vol, *along = nullptr;
-    if (scratch) {
-        float *ac = box.planar ? nullptr : scratch, *al = box.planar ? scratch : scratch + 2 * voxels;
+    const bool pairs = copies == ForwardCopies::Pairs;
+    if (copies != ForwardCopies::None) {
+        float *ac = pairs ? scratch : nullptr, *al = pairs ? scratch + 2 * voxels : scratch;
         long long grid = static_cast<long long>((box.nx + 31) / 32) * ((box.ny + 31) / 32) * box.nz;
         if (grid > static_cast<long long>(num_sms) * 64) grid = static_cast<long long>(num_sms) * 64;
-        if (box.planar)
+        if (!pairs)
             arrange_grid_kernel<false><<<static_cast<unsigned>(grid), dim3(32, 8), 0, s>>>(vol, box.nx, box.ny, box.nz, ac, al);
         else
             arrange_grid_kernel<true><<<static_cast<unsigned>(grid), dim3(32, 8), 0, s>>>(vol, box.nx, box.ny, box.nz, ac, al);
-        if (!box.planar) across = ac;
+        if (pairs) across = ac;
         along = al;
     }
     const int bx = nr >= 8 ? 32 : nr >= 4 ? 64 : nr >= 2 ? 128 : 256, by = 256 / bx;
@@ -442,15 +462,35 @@ void launch_forward(const ProjView *views, int kind, int nv, int nr, int nc, dou
                                                          step_vox, bx, out);
     };
     if (box.planar) go(forward_kernel<true, false, long long>);
-    else if (!scratch) go(forward_kernel<false, false, long long>);
+    else if (!pairs) go(forward_kernel<false, false, long long>);
     else if (8 * voxels < (1LL << 32)) go(forward_kernel<false, true, unsigned>);
     else go(forward_kernel<false, true, long long>);
 }
 
-long long forward_scratch_floats(const VolBox &box)
+ForwardCopies forward_copies(const VolBox &box, const ProjView *views, int kind, int nv, int nr, int nc,
+                             float step_vox)
 {
     const long long voxels = static_cast<long long>(box.nx) * box.ny * box.nz;
-    return voxels <= kCopyVoxels ? 0 : voxels * (box.planar ? 1 : 4);
+    if (voxels <= kCopyVoxels) return ForwardCopies::None;
+    if (box.planar) return ForwardCopies::Along;
+    if (16 * voxels <= kSmallCopies) return ForwardCopies::Pairs;
+    const double h = step_vox * std::min(box.w[0], std::min(box.w[1], box.w[2]));
+    const double samples = std::max(box.nx * box.w[0], box.ny * box.w[1]) / h * nr * nc;  // of a view
+    double along_x = 0.0, others = 0.0;
+    for (int v = 0; v < nv; ++v) {
+        const bool parallel = kind == GCT_GEOM_PARALLEL_2D || kind == GCT_GEOM_CONE_PARALLEL;
+        const double dy = std::fabs(parallel ? std::sin(views[v].extra) : views[v].ew[1]) * h / box.w[1];
+        (dy < 0.1 ? along_x : others) += samples;
+    }
+    const double pairs = kSaveX * along_x + kPairsSave * others - kCopyCall - kPairsVoxel * voxels;
+    const double along = kSaveX * along_x - kCopyCall - kAlongVoxel * voxels;
+    return std::max(pairs, along) <= 0.0 ? ForwardCopies::None : pairs >= along ? ForwardCopies::Pairs : ForwardCopies::Along;
+}
+
+long long forward_copy_floats(const VolBox &box, ForwardCopies copies)
+{
+    const long long voxels = static_cast<long long>(box.nx) * box.ny * box.nz;
+    return copies == ForwardCopies::Pairs ? 4 * voxels : copies == ForwardCopies::Along ? voxels : 0;
 }
 
 }  // namespace gct

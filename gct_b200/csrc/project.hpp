@@ -28,11 +28,16 @@ void launch_phantom(const ProjView *views, int kind, int nv, int nr, int nc, dou
                     const gct_ellipsoid *ell, int ne, bool planar, float *out, int num_sms,
                     cudaStream_t s);
 
-// scratch: room for forward_scratch_floats() floats, the copies of the grid that the rays read (made
-// here on the stream), or NULL: the rays read the grid itself, slower.
-long long forward_scratch_floats(const VolBox &box);
+// Copies of the grid that the rays of a call read: the grid with x and y exchanged for the views whose rays
+// run along x (Along), or that and the grid itself as (z, z + 1) pairs (Pairs, 3D grids).
+enum class ForwardCopies { None, Along, Pairs };
+// The copies that save the rays of the call more time than they take; views: on the host.
+ForwardCopies forward_copies(const VolBox &box, const ProjView *views, int kind, int nv, int nr, int nc,
+                             float step_vox);
+long long forward_copy_floats(const VolBox &box, ForwardCopies copies);
+// scratch: room for forward_copy_floats() floats; the copies are made there on the stream.
 void launch_forward(const ProjView *views, int kind, int nv, int nr, int nc, double du, double dv,
-                    const float *vol, float *scratch, const VolBox &box, float step_vox, float *out, int num_sms,
-                    cudaStream_t s);
+                    const float *vol, ForwardCopies copies, float *scratch, const VolBox &box, float step_vox, float *out,
+                    int num_sms, cudaStream_t s);
 
 }  // namespace gct
