@@ -625,7 +625,7 @@ void run_backproject_sym(gct_fdk_plan *p, const StackRef &st, float *vol, int b_
               : 0;
     launch_split(p, ba, chunk, s, [&](const gct::BpArgs &b) {
         gct::launch_backproject_sym(b, static_cast<int>(p->family), p->opts.storage, p->zpt_sym, p->bx_sym,
-                                    p->by_sym, s);
+                                    p->by_sym, p->num_sms, s);
         cuda_check(cudaGetLastError(), "backprojection kernel launch");
     });
 }

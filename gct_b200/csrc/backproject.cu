@@ -908,6 +908,20 @@ __global__ void __launch_bounds__(256) bp_sym_kernel(BpArgs a)
                              a.accumulate ? kBpAccumulate : kBpStore, s_coef, s_w, s_cls);
 }
 
+// bp_sym_kernel of the parallel kinds and arcs with FP16 quads, 8 voxels, in fewer registers: 96 instead of 108, ten
+// blocks of 64 threads per SM instead of nine, and 80 instead of 128, twelve instead of eight. A wave of it takes
+// longer (parallel 2 to 4 %, arcs up to half), so it is taken where it needs fewer by more than that (launch_sym_q).
+template <int FAMILY, class Q>
+__global__ void __maxnreg__(FAMILY == 0 ? 96 : 80) bp_sym_dense_kernel(BpArgs a)
+{
+    __shared__ float4 s_coef[kViewsPerChunk * kC / 4];
+    __shared__ float4 s_w[kViewsPerChunk];
+    __shared__ int s_cls[kViewsPerChunk];
+    sym_tile<FAMILY, Q, 8>(a, blockIdx.x * blockDim.x, blockIdx.y * blockDim.y, blockIdx.z * 8, blockDim.x, blockDim.y,
+                           threadIdx.y * blockDim.x + threadIdx.x, blockDim.x * blockDim.y,
+                           a.accumulate ? kBpAccumulate : kBpStore, s_coef, s_w, s_cls);
+}
+
 // The view-split launch of bp_sym_kernel (a.vchunk > 0, one-voxel-deep images): its own kernel, so
 // that the whole-volume kernel keeps its register allocation (the local copy of the arguments
 // here took it from 128 to 102 registers, and 34.8 to 42.5 ms at 512^3 / 720 views).
@@ -925,7 +939,7 @@ __global__ void __launch_bounds__(256) bp_sym_split_kernel(BpArgs a)
 }
 
 template <int FAMILY, class Q>
-void launch_sym_q(const BpArgs &a, int zpt, int bx, int by, cudaStream_t s)
+void launch_sym_q(const BpArgs &a, int zpt, int bx, int by, int num_sms, cudaStream_t s)
 {
     const int h = a.nx / 2;
     const dim3 block(bx, by);
@@ -944,7 +958,22 @@ void launch_sym_q(const BpArgs &a, int zpt, int bx, int by, cudaStream_t s)
         case 1: bp_sym_kernel<FAMILY, Q, 1><<<grid, block, 0, s>>>(a); break;
         case 2: bp_sym_kernel<FAMILY, Q, 2><<<grid, block, 0, s>>>(a); break;
         case 4: bp_sym_kernel<FAMILY, Q, 4><<<grid, block, 0, s>>>(a); break;
-        default: bp_sym_kernel<FAMILY, Q, 8><<<grid, block, 0, s>>>(a); break;
+        default:
+            if constexpr (FAMILY != 1 && sizeof(typename LerpOf<Q>::type::S) == 8) {
+                // 400 x 400 x 16, 720 views, 1.3 detector samples a voxel: parallel 1.27 ms in two waves, 0.91 in one,
+                // arcs 1.46 and 1.26; 208 x 208 x 64, 180 views, two waves either way: parallel 0.306 and 0.33
+                const long long blocks = static_cast<long long>(grid.x) * grid.y * grid.z;
+                const auto waves = [&](int regs) {
+                    const long long wave = 65536LL / (regs * static_cast<long long>(bx) * by) * num_sms;
+                    return (blocks + wave - 1) / wave;
+                };
+                if (FAMILY == 0 ? waves(96) < waves(112) : 1.5 * waves(80) < waves(128)) {
+                    bp_sym_dense_kernel<FAMILY, Q><<<grid, block, 0, s>>>(a);
+                    break;
+                }
+            }
+            bp_sym_kernel<FAMILY, Q, 8><<<grid, block, 0, s>>>(a);
+            break;
     }
 }
 
@@ -1132,16 +1161,17 @@ void launch_reduce_partials(const float *part, int nparts, long long n, float *v
                                                                                       accumulate ? 1 : 0);
 }
 
-void launch_backproject_sym(const BpArgs &a, int family, int storage, int zpt, int bx, int by, cudaStream_t s)
+void launch_backproject_sym(const BpArgs &a, int family, int storage, int zpt, int bx, int by, int num_sms,
+                            cudaStream_t s)
 {
     if (storage == 0) {
-        if (family == 0) launch_sym_q<0, QuadF32>(a, zpt, bx, by, s);
-        else if (family == 1) launch_sym_q<1, QuadF32>(a, zpt, bx, by, s);
-        else launch_sym_q<2, QuadF32>(a, zpt, bx, by, s);
+        if (family == 0) launch_sym_q<0, QuadF32>(a, zpt, bx, by, num_sms, s);
+        else if (family == 1) launch_sym_q<1, QuadF32>(a, zpt, bx, by, num_sms, s);
+        else launch_sym_q<2, QuadF32>(a, zpt, bx, by, num_sms, s);
     } else {
-        if (family == 0) launch_sym_q<0, QuadF16>(a, zpt, bx, by, s);
-        else if (family == 1) launch_sym_q<1, QuadF16>(a, zpt, bx, by, s);
-        else launch_sym_q<2, QuadF16>(a, zpt, bx, by, s);
+        if (family == 0) launch_sym_q<0, QuadF16>(a, zpt, bx, by, num_sms, s);
+        else if (family == 1) launch_sym_q<1, QuadF16>(a, zpt, bx, by, num_sms, s);
+        else launch_sym_q<2, QuadF16>(a, zpt, bx, by, num_sms, s);
     }
 }
 

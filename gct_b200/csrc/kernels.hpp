@@ -117,7 +117,8 @@ void launch_backproject(const BpArgs &a, int family, int storage, bool z_affine,
 // Quarter-turn form (a.sym != 0, z-affine geometries, nx == ny even): threads cover the first
 // quadrant of (x, y) columns; each evaluates the detector coordinates of its column once per base
 // view and accumulates them into the column's four quarter-turn images from the four partner views.
-void launch_backproject_sym(const BpArgs &a, int family, int storage, int zpt, int bx, int by, cudaStream_t s);
+void launch_backproject_sym(const BpArgs &a, int family, int storage, int zpt, int bx, int by, int num_sms,
+                            cudaStream_t s);
 
 // Planar kinds over row pairs (rows.cu): views [a.v_begin, a.v_begin + a.v_count) into the image.
 // a.quads, a.qview: the pairs and the entries per view; a.sym, a.quarter: quarter-turn plans, whose
