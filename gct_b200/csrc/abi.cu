@@ -598,7 +598,7 @@ void run_backproject(gct_fdk_plan *p, const StackRef &st, float *vol, int v_begi
               : 0;
     launch_split(p, ba, chunk, s, [&](const gct::BpArgs &b) {
         gct::launch_backproject(b, static_cast<int>(p->family), p->opts.storage, p->z_affine, p->zpt, p->bx, p->by,
-                                s);
+                                p->num_sms, s);
         cuda_check(cudaGetLastError(), "backprojection kernel launch");
     });
 }

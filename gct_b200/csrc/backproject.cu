@@ -580,8 +580,31 @@ __global__ void __launch_bounds__(256) bp_mirror_kernel(BpArgs a)
                                              a.accumulate ? kBpAccumulate : kBpStore);
 }
 
+// Whole-volume launches of bp_kernel for FP32 arcs, 16 voxels, in 56 registers: eighteen blocks of 64 threads per SM
+// where sixteen fit. Taken where it saves a wave (400 x 400 x 16, 720 views, 1.3 detector samples a voxel 2.70 ms in two
+// waves, 1.79 in one).
+template <class Q>
+__global__ void __maxnreg__(56) bp_arc_dense_kernel(BpArgs a)
+{
+    __shared__ float4 s_coef[kViewsPerChunk * kC / 4];
+    __shared__ int s_cls[kViewsPerChunk];
+    __shared__ BlockBox s_box;
+    const int i = blockIdx.x * blockDim.x + threadIdx.x, j = blockIdx.y * blockDim.y + threadIdx.y;
+    bp_column<2, Q, 16, true, 1>(a, i, j, blockIdx.z * 16, i < a.nx && j < a.ny, kViewsPerChunk, s_coef, s_cls, &s_box,
+                                 threadIdx.y * blockDim.x + threadIdx.x, blockDim.x * blockDim.y,
+                                 a.accumulate ? kBpAccumulate : kBpStore);
+}
+
+// Waves of a launch of a kernel that takes `regs` registers (a multiple of 8) per thread.
+long long launch_waves(dim3 grid, dim3 block, int regs, int num_sms)
+{
+    const long long wave = 65536LL / (static_cast<long long>(regs) * block.x * block.y) * num_sms;
+    const long long blocks = static_cast<long long>(grid.x) * grid.y * grid.z;
+    return wave > 0 ? (blocks + wave - 1) / wave : blocks;
+}
+
 template <int FAMILY, class Q, int ZPT>
-void launch_zpt(const BpArgs &a, bool z_affine, dim3 grid, dim3 block, cudaStream_t s)
+void launch_zpt(const BpArgs &a, bool z_affine, dim3 grid, dim3 block, int num_sms, cudaStream_t s)
 {
     if constexpr (FAMILY != 2 && ZPT % 2 == 0) {
         if (a.mirror) {
@@ -595,6 +618,13 @@ void launch_zpt(const BpArgs &a, bool z_affine, dim3 grid, dim3 block, cudaStrea
             return;
         }
     }
+    if constexpr (FAMILY == 2 && ZPT == 16 && sizeof(typename LerpOf<Q>::type::S) == 16) {
+        if (z_affine && !a.quarter && a.vchunk <= 0 && !a.slice_views &&
+            launch_waves(grid, block, 56, num_sms) < launch_waves(grid, block, 64, num_sms)) {
+            bp_arc_dense_kernel<Q><<<grid, block, 0, s>>>(a);
+            return;
+        }
+    }
     if (a.quarter)  // interleaved partner views: quarter-turn plans, which are z-affine
         bp_kernel<FAMILY, Q, ZPT, true, 4><<<grid, block, 0, s>>>(a);
     else if (z_affine || FAMILY == 0)
@@ -604,18 +634,18 @@ void launch_zpt(const BpArgs &a, bool z_affine, dim3 grid, dim3 block, cudaStrea
 }
 
 template <int FAMILY, class Q>
-void launch_q(const BpArgs &a, bool z_affine, int zpt, int bx, int by, cudaStream_t s)
+void launch_q(const BpArgs &a, bool z_affine, int zpt, int bx, int by, int num_sms, cudaStream_t s)
 {
     const dim3 block(bx, by);
     const int nz = a.mirror ? a.nz / 2 : a.nz;  // mirror launches cover the lower half
     const unsigned gz = a.vchunk > 0 ? (a.v_count + a.vchunk - 1) / a.vchunk : (nz + zpt - 1) / zpt;
     const dim3 grid((a.nx + bx - 1) / bx, (a.ny + by - 1) / by, gz);
     switch (zpt) {
-        case 1: launch_zpt<FAMILY, Q, 1>(a, z_affine, grid, block, s); break;
-        case 2: launch_zpt<FAMILY, Q, 2>(a, z_affine, grid, block, s); break;
-        case 4: launch_zpt<FAMILY, Q, 4>(a, z_affine, grid, block, s); break;
-        case 8: launch_zpt<FAMILY, Q, 8>(a, z_affine, grid, block, s); break;
-        default: launch_zpt<FAMILY, Q, 16>(a, z_affine, grid, block, s); break;
+        case 1: launch_zpt<FAMILY, Q, 1>(a, z_affine, grid, block, num_sms, s); break;
+        case 2: launch_zpt<FAMILY, Q, 2>(a, z_affine, grid, block, num_sms, s); break;
+        case 4: launch_zpt<FAMILY, Q, 4>(a, z_affine, grid, block, num_sms, s); break;
+        case 8: launch_zpt<FAMILY, Q, 8>(a, z_affine, grid, block, num_sms, s); break;
+        default: launch_zpt<FAMILY, Q, 16>(a, z_affine, grid, block, num_sms, s); break;
     }
 }
 
@@ -962,11 +992,7 @@ void launch_sym_q(const BpArgs &a, int zpt, int bx, int by, int num_sms, cudaStr
             if constexpr (FAMILY != 1 && sizeof(typename LerpOf<Q>::type::S) == 8) {
                 // 400 x 400 x 16, 720 views, 1.3 detector samples a voxel: parallel 1.27 ms in two waves, 0.91 in one,
                 // arcs 1.46 and 1.26; 208 x 208 x 64, 180 views, two waves either way: parallel 0.306 and 0.33
-                const long long blocks = static_cast<long long>(grid.x) * grid.y * grid.z;
-                const auto waves = [&](int regs) {
-                    const long long wave = 65536LL / (regs * static_cast<long long>(bx) * by) * num_sms;
-                    return (blocks + wave - 1) / wave;
-                };
+                const auto waves = [&](int regs) { return launch_waves(grid, block, regs, num_sms); };
                 if (FAMILY == 0 ? waves(96) < waves(112) : 1.5 * waves(80) < waves(128)) {
                     bp_sym_dense_kernel<FAMILY, Q><<<grid, block, 0, s>>>(a);
                     break;
@@ -1214,16 +1240,16 @@ void launch_backproject_queue(const BpItem *items, const BpWork *work, int n_wor
 }
 
 void launch_backproject(const BpArgs &a, int family, int storage, bool z_affine, int zpt, int bx,
-                        int by, cudaStream_t s)
+                        int by, int num_sms, cudaStream_t s)
 {
     if (storage == 0) {
-        if (family == 0) launch_q<0, QuadF32>(a, z_affine, zpt, bx, by, s);
-        else if (family == 1) launch_q<1, QuadF32>(a, z_affine, zpt, bx, by, s);
-        else launch_q<2, QuadF32>(a, z_affine, zpt, bx, by, s);
+        if (family == 0) launch_q<0, QuadF32>(a, z_affine, zpt, bx, by, num_sms, s);
+        else if (family == 1) launch_q<1, QuadF32>(a, z_affine, zpt, bx, by, num_sms, s);
+        else launch_q<2, QuadF32>(a, z_affine, zpt, bx, by, num_sms, s);
     } else {
-        if (family == 0) launch_q<0, QuadF16>(a, z_affine, zpt, bx, by, s);
-        else if (family == 1) launch_q<1, QuadF16>(a, z_affine, zpt, bx, by, s);
-        else launch_q<2, QuadF16>(a, z_affine, zpt, bx, by, s);
+        if (family == 0) launch_q<0, QuadF16>(a, z_affine, zpt, bx, by, num_sms, s);
+        else if (family == 1) launch_q<1, QuadF16>(a, z_affine, zpt, bx, by, num_sms, s);
+        else launch_q<2, QuadF16>(a, z_affine, zpt, bx, by, num_sms, s);
     }
 }
 

@@ -112,7 +112,7 @@ void launch_reduce_partials(const float *part, int nparts, long long n, float *v
 // Voxel-driven backprojection. family: 0 affine, 1 projective, 2 arc. storage: 0 f32, 1 f16.
 // z_affine selects the column kernel (u and the denominator constant along z).
 void launch_backproject(const BpArgs &a, int family, int storage, bool z_affine, int zpt,
-                        int bx, int by, cudaStream_t s);
+                        int bx, int by, int num_sms, cudaStream_t s);
 
 // Quarter-turn form (a.sym != 0, z-affine geometries, nx == ny even): threads cover the first
 // quadrant of (x, y) columns; each evaluates the detector coordinates of its column once per base
