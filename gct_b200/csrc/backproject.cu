@@ -35,8 +35,8 @@ constexpr float kShift = 12582912.0f;  // 1.5 * 2^23
 constexpr int kShiftBits = 0x4B400000;  // bit pattern of kShift
 
 // Coefficient layouts (per view, kCoefPerView floats):
-//  affine     : [0..2] u0, ui, uj; [3..4] v0, vk; [5] wscale; [6..7] vi, vj (zero except for the
-//               transposed one-row detector, where v is the detector coordinate)
+//  affine     : [0..2] u0, ui, uj; [3..4] v0, vk; [5] wscale; [6..7] vi, vj, always zero: the
+//               row coordinate does not depend on the column
 //  projective : [0..3] U numerator; [4..7] V numerator; [8..11] denominator D; [12] wscale
 //               u = U/D, v = V/D, weight = wscale / D^2
 //  arc        : [0..3] A = e_u.d; [4..7] B = e_w.d; [8..11] T = e_v.d; [12] 1/dgamma; [13] c0;
@@ -47,8 +47,8 @@ constexpr int kShiftBits = 0x4B400000;  // bit pattern of kShift
 __device__ __forceinline__ int wscale_slot(int family) { return family == 0 ? 5 : family == 1 ? 12 : 16; }
 
 // Quad loads ask L2 for whole 256 bytes: a block's next rows and views' neighbours lie there, and fewer
-// gathers wait for DRAM (FP32 quads 512^3 / 720 views 71.4 -> 70.2 ms, 256^3 / 360 views 4.48 -> 4.40; FP16 short
-// scan 34.8 -> 34.6).
+// gathers wait for DRAM (FP32 quads 512^3 / 720 views 71.4 -> 70.2 ms, 256^3 / 360 views 4.48 -> 4.40; FP16 within
+// what runs differ).
 __device__ __forceinline__ uint2 ldg_quad(const uint2 *p)
 {
     uint2 r;

@@ -74,7 +74,6 @@ gct_view_geom view_from_projection_matrix(const ProjMatrix &pm);
 std::vector<double> ramp_taps(gct_geom_kind kind, const gct_detector &det_row,
                               const gct_filt_params &fp);
 
-// Parker (redundancy) weights [view][col]; see gct_parker_weights in gct_fdk.h.
 // Redundancy weights of a scan: one constant (gamma empty), or Parker's windows of the fan angles gamma
 // [col] and the relative view angles rel [view] over the range phi.
 struct ParkerRule {
@@ -82,6 +81,7 @@ struct ParkerRule {
     std::vector<double> gamma, rel;
 };
 ParkerRule parker_rule(const gct_ct_geom &g, const RotationInfo &ri);
+// Parker (redundancy) weights [view][col]; see gct_parker_weights in gct_fdk.h.
 std::vector<double> parker_table(const gct_ct_geom &g, const RotationInfo &ri);
 
 // Smallest power of two L for which an L-point circular convolution of N samples with the

@@ -50,9 +50,9 @@ __host__ __device__ inline void quad_layout(long long v, long long qview, int qu
     }
 }
 
-// Row pairs: the stack of planar kinds (1D parallel, fan line, fan arc), whose views are one row. Entry c of a view, for c in [-2, nc + 2), is (y[c], y[c + 1] - y[c]), for the
-// parallel kind ((y[c] + y[c + 1]) / 2, y[c + 1] - y[c]), with zeros outside the row, as float2 or half2
-// (scaled as the quads); views follow each other nc + 4 entries apart, or (FP16 lines with
+// Row pairs: the stack of planar kinds (1D parallel, fan line, fan arc), whose views are one row. Entry c
+// of a view, for c in [-2, nc + 2), is (y[c], y[c + 1] - y[c]), for the parallel kind
+// ((y[c] + y[c + 1]) / 2, y[c + 1] - y[c]), with zeros outside the row, as float2 or half2 (scaled as the quads); views follow each other nc + 4 entries apart, or (FP16 lines with
 // the quarter-turn symmetry) partner views are interleaved as in quad_layout. With FP16 storage the
 // fans keep quads in two cases: arcs, whose blends round the column fraction to half precision, which
 // turns last-bit differences of the angle into differences of a 2048th sample, so they stay with

@@ -200,7 +200,8 @@ void start(gct_fdk_server *s, Request *r)
     r->proj_dev = reinterpret_cast<float *>(base);
     unsigned char *ws = base + gct::Arena::round_up(r->proj_bytes);
     r->vol_dev = reinterpret_cast<float *>(ws + gct::Arena::round_up(r->plan->workspace_bytes()));
-    // quarter-turn plans keep their interleaved partner stacks (the quarter-turn queue class)
+    // quarter-turn plans keep their interleaved partner stacks (the quarter-turn queue class), but for row
+    // pairs: the planar queue takes view-major ones
     r->st = stack_of(r->plan, ws, r->plan->rows);
     for (cudaEvent_t *e : {&r->e_in, &r->e_prep, &r->e_out})
         cuda_check(cudaEventCreateWithFlags(e, cudaEventDisableTiming), "request event");

@@ -181,8 +181,12 @@ enum {
 typedef struct gct_fdk_opts {
     int32_t filter;        /* GCT_FILTER_* */
     int32_t storage;       /* GCT_STORAGE_* */
-    int32_t z_per_thread;  /* backprojection voxels per thread along z; 0 = tuned default */
-    int32_t block_x;       /* backprojection block shape; 0 = tuned default */
+    /* Backprojection voxels per thread along z and block shape; 0 = tuned default. Plans of one-row
+     * detectors whose filtered views are rows (1D parallel; FP32 fans; FP16 fan lines with the FFT filter)
+     * have a fixed shape: the values are checked there and have no effect. Spiral scans take 4, 8 or 16
+     * slices per thread, else one. */
+    int32_t z_per_thread;
+    int32_t block_x;
     int32_t block_y;
     int32_t symmetry;      /* GCT_SYMMETRY_* */
     int32_t scan;          /* GCT_SCAN_* */
