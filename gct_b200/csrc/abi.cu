@@ -300,9 +300,9 @@ void build_plan(gct_fdk_plan *p, const gct_ct_geom *g, const gct_vol_geom *vol,
     // 256 x 256 x 256 3.5 against 4.2, 512 x 512 x 256 11.8 against 12.8).
     // Of flat panels: a wave of blocks with 16 voxels (16 blocks of 64 threads per SM) takes 1.9 times as long
     // as one with 8 (465 and 245 us with 240 views), so 8 where that fills the device better (a tie goes to
-    // 16: 300 x 300 x 211, 100 views 1.46 against 1.39 ms). 240 views: 128 x 128 x 32 0.21 (8) against 0.35 ms (16), 224 x 224 x 56 0.73 against 0.83, 320 x 320 x 80 1.62
-    // against 1.81, 253 x 241 x 187 (short scan, 247 views) 2.85 against 2.96; the other way 192^3 1.60 against 1.42,
-    // 256^3 3.47 against 3.23, 512^3 27.2 against 25.8.
+    // 16: 300 x 300 x 211, 100 views 1.46 against 1.39 ms). 240 views: 128 x 128 x 32 0.21 (8) against 0.35 ms
+    // (16), 224 x 224 x 56 0.73 against 0.83, 320 x 320 x 80 1.62 against 1.81, 253 x 241 x 187 (short scan, 247 views)
+    // 2.85 against 2.96; the other way 192^3 1.60 against 1.42, 256^3 3.47 against 3.23, 512^3 27.2 against 25.8.
     // Arcs keep 16 (381 x 379 x 61, 577 views 5.4 ms, 5.6 with 8).
     const auto waves = [&](int z) {
         const long long blocks = static_cast<long long>((p->kx + p->bx - 1) / p->bx) *

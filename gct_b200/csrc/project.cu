@@ -25,10 +25,10 @@ constexpr long long kCopyVoxels = 1 << 14;
 // cost next to nothing (48^3 voxels, 4 views of 64 x 64 and more: 0 to 15 % less time with them); larger ones cost
 // 0.5 ms and 18 us per million voxels, the exchanged grid alone 5 us. A million samples of rays along x, within
 // the tenth of a voxel of y per step that keeps the warp from marching in step, take 15 to 24 us longer in the
-// grid itself than in either copy (every gather touches 32 lines); others
-// take 0.8 us longer than in the pairs. Without / exchanged grid / pairs, ms a call: 2 views of 64 x 64 through 512^3
-// 1.4 / - / 4.9, of 256 x 256 5.0 / 3.3 / 5.2, of 512 x 512 10.4 / 3.4 / 5.8; 8 views of 96 x 96 through 96^3 1.0 / - / 1.4,
-// 180 of 160 x 160 5.3 / - / 3.3; 192^3, 16 views of 256 x 256, half-voxel steps 2.7 / - / 2.3, whole ones 1.8 / - / 2.0.
+// grid itself than in either copy (every gather touches 32 lines); others take 0.8 us longer than in the
+// pairs. Without / exchanged grid / pairs, ms a call: 2 views of 64 x 64 through 512^3 1.4 / - / 4.9, of
+// 256 x 256 5.0 / 3.3 / 5.2, of 512 x 512 10.4 / 3.4 / 5.8; 8 views of 96 x 96 through 96^3 1.0 / - / 1.4, 180 of
+// 160 x 160 5.3 / - / 3.3; 192^3, 16 views of 256 x 256, half-voxel steps 2.7 / - / 2.3, whole ones 1.8 / - / 2.0.
 constexpr long long kSmallCopies = 2 << 20;
 constexpr double kCopyCall = 500.0, kPairsVoxel = 18e-6, kAlongVoxel = 5e-6;
 constexpr double kSaveX = 21e-6, kPairsSave = 0.8e-6;
